@@ -258,6 +258,7 @@ template <class R> class Engine {
     struct GraphEntry {
         int kk, nsys, zpar;
         double tol;
+        bool blocked;
         cudaGraphExec_t exec;
     };
     std::vector<GraphEntry> graphs_;
@@ -267,6 +268,11 @@ template <class R> class Engine {
     int enqueue_front(int kk, int nsys, long *matvecs);
     int enqueue_krylov(int kk, int nsys, double tol, long *matvecs);
     int enqueue_back(int kk, int nsys, bool join);
+    // Blocked Krylov steps: blocked_ is set around a refined complex64 cycle while blocks_on_ (from
+    // refine_setup until a system's block turns out ill-conditioned).
+    bool blocked_ = false, blocks_on_ = true;
+    bool blocked_ok(int kk, int nsys) const;
+    int enqueue_krylov_blocked(int kk, int nsys, double tol, long *matvecs);
     // lockstep (many-operator) form: the cycle the last multi_front set up
     int mf_kk_ = 0, mf_nsys_ = 0;
     bool mf_ran_ = false;       // a cycle ran since the last multi_select

@@ -35,6 +35,17 @@ __device__ __forceinline__ double2 to_d(dfc a) { return make_double2((double)a.x
 
 template <class C> __device__ __forceinline__ C czero() { C z; z.x = 0; z.y = 0; return z; }
 
+// the value of a matrix entry in type C, rounded on the host as the stored arrays are
+template <class C> C host_value(double2 a);
+template <> float2 host_value<float2>(double2 a) { return make_float2((float)a.x, (float)a.y); }
+template <> double2 host_value<double2>(double2 a) { return a; }
+template <> dfc host_value<dfc>(double2 a) {
+    dfc c;
+    c.x = dfr(a.x);
+    c.y = dfr(a.y);
+    return c;
+}
+
 // a * b + c in the working real type
 __device__ __forceinline__ float rfma(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double rfma(double a, double b, double c) { return ::fma(a, b, c); }
@@ -95,6 +106,20 @@ template <class C> __device__ __forceinline__ void cfms_r(C &acc, C a, C b, bool
     } else {
         cfms(acc, a, b);
     }
+}
+// What an operator kernel does with its row sum: y = A x; the pending normalisation y = a (A x), v = a x;
+// or the shifted product y = s (A x - t x).  (k_spmm tests at run time instead: with the mode as a template
+// argument its loads were scheduled worse, 520 against 380 us for 64 shifted products at 96^3.)
+enum OpMode { OP_PLAIN, OP_SCALE, OP_SHIFT };
+// sigma (acc - t x): the epilogue of a shifted product (blocked Krylov steps)
+template <class C, class R> __device__ __forceinline__ C shifted(C acc, C x, C t, R sigma) {
+    cfms(acc, t, x);
+    acc.x = acc.x * sigma;
+    acc.y = acc.y * sigma;
+    return acc;
+}
+template <class C> __device__ __forceinline__ C shift_of(const SysState &st) {
+    return from_d<C>(make_double2((double)st.bs_tr, (double)st.bs_ti));
 }
 // acc += conj(a) * b
 template <class C> __device__ __forceinline__ void cdotacc(C &acc, C a, C b) {
@@ -3561,9 +3586,9 @@ template <class C> __device__ __forceinline__ C cadd(C a, C b) {
     return r;
 }
 constexpr int ST_ZC = 8;
-template <class R>
-__global__ void __launch_bounds__(NT) k_stencil(int nx, int ny, int nz, double2 dd, double2 wxd, double2 wyd,
-                                                double2 wzd, const typename CT<R>::t *__restrict__ x0, size_t strideX,
+template <class R, int MODE>
+__global__ void __launch_bounds__(NT) k_stencil(int nx, int ny, int nz, typename CT<R>::t d,
+                                                typename CT<R>::t wx, typename CT<R>::t wy, typename CT<R>::t wz, const typename CT<R>::t *__restrict__ x0, size_t strideX,
                                                 typename CT<R>::t *__restrict__ y0, size_t strideY,
                                                 const int *__restrict__ act, const SysState *__restrict__ scale,
                                                 typename CT<R>::t *__restrict__ vout0, size_t strideVO) {
@@ -3572,14 +3597,14 @@ __global__ void __launch_bounds__(NT) k_stencil(int nx, int ny, int nz, double2 
     const C *x = x0 + (size_t)sys * strideX;
     C *y = y0 + (size_t)sys * strideY;
     // pending normalisation, as in k_spmm: x is w, y = a (A w), vout = a w
-    const R al = scale ? (R)scale[sys].alpha : R(1.0);
-    const bool brk = scale && scale[sys].broken;
-    C *vout = scale ? vout0 + (size_t)sys * strideVO : nullptr;
+    const R al = MODE == OP_SHIFT ? (R)(double)scale[sys].bs_sigma : MODE == OP_SCALE ? (R)scale[sys].alpha : R(1.0);
+    const bool brk = MODE == OP_SCALE && scale[sys].broken;
+    const C th = MODE == OP_SHIFT ? shift_of<C>(scale[sys]) : czero<C>();
+    C *vout = MODE == OP_SCALE ? vout0 + (size_t)sys * strideVO : nullptr;
     const int tilesx = (nx + 31) / 32;
     const int ix = (blockIdx.x % tilesx) * 32 + (threadIdx.x & 31);
     const int iy = (blockIdx.x / tilesx) * 8 + (threadIdx.x >> 5);
     if (ix >= nx || iy >= ny) return;
-    const C d = from_d<C>(dd), wx = from_d<C>(wxd), wy = from_d<C>(wyd), wz = from_d<C>(wzd);
     const long plane = (long)nx * ny;
     const int z0 = blockIdx.y * ST_ZC, z1 = min(nz, z0 + ST_ZC);
     long idx = (long)iy * nx + ix + (long)z0 * plane;
@@ -3597,7 +3622,7 @@ __global__ void __launch_bounds__(NT) k_stencil(int nx, int ny, int nz, double2 
         cfma(acc, wx, sx);
         cfma(acc, wy, sy);
         cfma(acc, wz, cadd(below, above));
-        if (vout) {
+        if (MODE == OP_SCALE) {
             C v = cur;
             v.x = v.x * al;
             v.y = v.y * al;
@@ -3605,6 +3630,8 @@ __global__ void __launch_bounds__(NT) k_stencil(int nx, int ny, int nz, double2 
             acc.y = acc.y * al;
             if (brk) v = czero<C>();
             vout[idx] = canon(v);
+        } else if (MODE == OP_SHIFT) {
+            acc = shifted(acc, cur, th, al);
         }
         y[idx] = canon(acc);
         below = cur;
@@ -3624,7 +3651,7 @@ __global__ void __launch_bounds__(NT) k_stencil(int nx, int ny, int nz, double2 
 // lies outside the grid is left out where the SELL kernels add a stored zero times x.  So both
 // forms give the same values for a matrix whose CSR rows are sorted and free of duplicates.
 constexpr int GR_ZC = 8;
-template <class R, int SG>
+template <class R, int SG, int MODE>
 __global__ void __launch_bounds__(NT) k_grid_spmm(int nx, int ny, int nz, int ngroups, int ntiles,
                                                   unsigned greal, const typename CT<R>::t *__restrict__ coef,
                                                   const typename CT<R>::t *__restrict__ x0, size_t strideX,
@@ -3650,6 +3677,7 @@ __global__ void __launch_bounds__(NT) k_grid_spmm(int nx, int ny, int nz, int ng
     C below[SG], cur[SG];
     R al[SG];      // pending normalisation factors, converted once (a double -> float conversion
     bool bk[SG];   // is an FP64-pipe instruction on GB300)
+    C th[SG];      // shifts of a shifted product
 #pragma unroll
     for (int g = 0; g < SG; ++g) {
         al[g] = R(1.0);
@@ -3658,7 +3686,11 @@ __global__ void __launch_bounds__(NT) k_grid_spmm(int nx, int ny, int nz, int ng
             xs[g] = x0 + (size_t)act[g0 + g] * strideX;
             below[g] = z0 > 0 ? xs[g][idx - plane] : czero<C>();
             cur[g] = xs[g][idx];
-            if (scale) {
+            th[g] = czero<C>();
+            if (MODE == OP_SHIFT) {
+                al[g] = (R)(double)scale[act[g0 + g]].bs_sigma;
+                th[g] = shift_of<C>(scale[act[g0 + g]]);
+            } else if (MODE == OP_SCALE) {
                 al[g] = (R)scale[act[g0 + g]].alpha;
                 bk[g] = scale[act[g0 + g]].broken != 0;
             }
@@ -3689,7 +3721,9 @@ __global__ void __launch_bounds__(NT) k_grid_spmm(int nx, int ny, int nz, int ng
                 if (yh) cfma_r(acc, apQ, x[idx + nx], rpQ);
                 if (zh) cfma_r(acc, apP, above, rpP);
                 const int sys = act[g0 + g];
-                if (scale) {   // pending normalisation, as in k_spmm
+                if (MODE == OP_SHIFT) {
+                    acc = shifted(acc, cur[g], th[g], al[g]);
+                } else if (MODE == OP_SCALE) {   // pending normalisation, as in k_spmm
                     C v = cur[g];
                     v.x = v.x * al[g];
                     v.y = v.y * al[g];
@@ -3709,7 +3743,7 @@ __global__ void __launch_bounds__(NT) k_grid_spmm(int nx, int ny, int nz, int ng
 // One system: two rows a thread (row r and r + NT of a 2*NT-row chunk), both rows' entries
 // loaded before any gather, so the two dependent trips (column index, then x) overlap across
 // the rows; rows wider than WMAX take the generic loop.
-template <class R>
+template <class R, int MODE>
 __global__ void __launch_bounds__(NT, 2) k_spmv2(int n, const int *__restrict__ slice_ptr, const int *__restrict__ cols,
                                               const typename CT<R>::t *__restrict__ vals,
                                               const typename CT<R>::t *__restrict__ x0, size_t strideX,
@@ -3722,9 +3756,10 @@ __global__ void __launch_bounds__(NT, 2) k_spmv2(int n, const int *__restrict__ 
     const int sys = act[0];
     const C *x = x0 + (size_t)sys * strideX;
     C *y = y0 + (size_t)sys * strideY;
-    // pending normalisation, as in k_spmm
-    const R al = scale ? (R)scale[sys].alpha : R(1.0);
-    const bool brk = scale && scale[sys].broken;
+    // pending normalisation or shifted product, as in k_spmm
+    const R al = MODE == OP_SHIFT ? (R)(double)scale[sys].bs_sigma : MODE == OP_SCALE ? (R)scale[sys].alpha : R(1.0);
+    const bool brk = MODE == OP_SCALE && scale[sys].broken;
+    const C th = MODE == OP_SHIFT ? shift_of<C>(scale[sys]) : czero<C>();
     const long rbase = (long)blockIdx.x * 2 * NT + threadIdx.x;
     C v[2][WMAX];
     int c[2][WMAX], width[2];
@@ -3767,7 +3802,9 @@ __global__ void __launch_bounds__(NT, 2) k_spmv2(int n, const int *__restrict__ 
                 acc = canon(acc);
             }
         }
-        if (scale) {
+        if (MODE == OP_SHIFT) {
+            acc = shifted(acc, x[row], th, al);
+        } else if (MODE == OP_SCALE) {
             C v = x[row];
             v.x = v.x * al;
             v.y = v.y * al;
@@ -3798,25 +3835,28 @@ __global__ void __launch_bounds__(NT) k_spmm(int n, const int *__restrict__ slic
     // basis entry v_s = a_s w_s goes to vout_s (a_s = state[s].alpha; zeros after a breakdown),
     // which spares the normalisation kernel its pass over w.  The factors are converted once per
     // CTA: a double -> float conversion per row and system would be an FP64-pipe instruction
-    // per element on GB300.
+    // per element on GB300.  Likewise the factors of the shifted product y_s = s (A x_s - t x_s).
     __shared__ R s_al[SG];
     __shared__ int s_bk[SG];
+    __shared__ C s_th[SG];
     if (scale && (int)threadIdx.x < ng) {
         const SysState &stt = scale[act[g0 + threadIdx.x]];
-        s_al[threadIdx.x] = (R)stt.alpha;
+        s_al[threadIdx.x] = vout0 ? (R)stt.alpha : (R)(double)stt.bs_sigma;
         s_bk[threadIdx.x] = stt.broken;
+        s_th[threadIdx.x] = shift_of<C>(stt);
     }
     __syncthreads();
     auto fin = [&](int g, int sys, long row, C acc, const C *x) {
         if (scale) {
             const R al = s_al[g];
             C v = x[row];
+            if (!vout0) cfms(acc, s_th[g], v);
             v.x = v.x * al;
             v.y = v.y * al;
             acc.x = acc.x * al;
             acc.y = acc.y * al;
             if (s_bk[g]) v = czero<C>();
-            vout0[(size_t)sys * strideVO + row] = canon(v);
+            if (vout0) vout0[(size_t)sys * strideVO + row] = canon(v);
         }
         y0[(size_t)sys * strideY + row] = canon(acc);
     };
@@ -3957,9 +3997,14 @@ __global__ void __launch_bounds__(NT) k_refine_update(int n, double2 *__restrict
     using C = typename CT<R>::t;
     const int s = act[blockIdx.y];
     const double sc = state[s].true_res;
+    const bool drop = state[s].ill != 0;   // the cycle's correction is not used
     double2 *x = x0 + (size_t)s * strideX;
     C *d = d0 + (size_t)s * strideD;
     for (long i = (long)blockIdx.x * NT + threadIdx.x; i < n; i += (long)gridDim.x * NT) {
+        if (drop) {
+            d[i] = czero<C>();
+            continue;
+        }
         C dv = d[i];
         double2 xv = x[i];
         if constexpr (std::is_same<C, float2>::value) {
@@ -4107,6 +4152,9 @@ struct Launch {
 };
 }  // namespace
 
+ProfScope::ProfScope(int kc, double bytes, cudaStream_t st, int nlaunch) : impl_(new Launch(kc, bytes, st, nlaunch)) {}
+ProfScope::~ProfScope() { delete static_cast<Launch *>(impl_); }
+int device_sm_count() { return num_sms(); }
 long long launch_count() { return g_launches.load(); }
 void profile_enable(bool on) { g_prof = on; }
 bool profile_enabled() { return g_prof; }
@@ -4218,6 +4266,8 @@ template <class K> void allow_smem(K kernel, size_t bytes) {
 }
 }  // namespace
 
+void block_allow_smem(const void *kernel, size_t bytes) { allow_smem(kernel, bytes); }
+
 // ----------------------------------------------------------------- scratch registry
 // Engines register their reduction scratch (pointer, doubles); the Gram-Schmidt launchers
 // skip any kernel variant whose partial sums would not fit, so no variant can overrun it.
@@ -4238,6 +4288,7 @@ void register_scratch(const void *p, size_t doubles) {
         if (e.first == p) { e.second = doubles; return; }
     g_scratch.emplace_back(p, doubles);
 }
+size_t scratch_size(const void *p) { return scratch_capacity(p); }
 void unregister_scratch(const void *p) {
     std::lock_guard<std::mutex> lk(g_scratch_mu);
     for (size_t i = 0; i < g_scratch.size(); ++i)
@@ -4279,16 +4330,19 @@ thread_local bool t_capturing = false;   // a stream capture is open on this thr
 // launches, because a batch sharing W is limited by re-reading W and favours other tiles.
 // Engines run their first two cycles eagerly, so every class they use is settled before a
 // cycle is captured into a CUDA graph.
-int bucket_of(int nsys, int qa) { return (nsys > 1 ? 1 : 0) + (qa > 0 ? 2 : 0); }
+int bucket_of(int nsys, int qa, int qb) {
+    // a batch against the shared vectors alone (the deflator of the blocked Krylov steps) is its own class
+    return (nsys > 1 ? 1 : 0) + (qa > 0 ? 2 : 0) + (nsys > 1 && qa > 0 && qb == 0 ? 4 : 0);
+}
 
 // A class is tuned on its first launch with at least 8 own-basis vectors (mid-cycle Krylov
 // steps, where the own part weighs as it does on average), or, for a single system, at least
 // 8 shared vectors (the deflation loop, which has no own part).
-bool representative(int nsys, int qa, int qb) { return qb >= 8 || (nsys == 1 && qa >= 8); }
+bool representative(int nsys, int qa, int qb) { return qb >= 8 || (qa >= 8 && (nsys == 1 || qb == 0)); }
 
 template <class F>
-int tuned_variant(int prec, int kernel, int n, int nsys, int qa, int nvar, cudaStream_t st, F &&run) {
-    const TuneKey key{prec, kernel, n, bucket_of(nsys, qa)};
+int tuned_variant(int prec, int kernel, int n, int nsys, int qa, int qb, int nvar, cudaStream_t st, F &&run) {
+    const TuneKey key{prec, kernel, n, bucket_of(nsys, qa, qb)};
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         for (auto &e : g_tuned)
@@ -4349,8 +4403,8 @@ std::string tune_report() {
         char buf[256];
         int len = snprintf(buf, sizeof buf, "%s %s n=%d %s %s: variant %d [",
                            e.key.prec == 4 ? "c64" : e.key.prec == 9 ? "df64" : "c128",
-                           e.key.kernel == 0 ? "projection" : "update", e.key.n,
-                           (e.key.bucket & 1) ? "batch" : "single", (e.key.bucket & 2) ? "shared" : "own", e.variant);
+                           e.key.kernel == 0 ? "projection" : e.key.kernel == 1 ? "update" : "deflator", e.key.n,
+                           (e.key.bucket & 1) ? "batch" : "single", (e.key.bucket & 4) ? "shared-only" : (e.key.bucket & 2) ? "shared" : "own", e.variant);
         out.append(buf, len);
         for (int v = 0; v < e.nvar; ++v) {
             len = snprintf(buf, sizeof buf, "%s%.4f", v ? " " : "", e.ms[v]);
@@ -4521,7 +4575,7 @@ int mdot_dispatch(int v, int n, const typename CT<R>::t *segA, int qa, const typ
                 {
                     std::lock_guard<std::mutex> lk(g_tune_mu);
                     for (auto &e : g_tuned)
-                        if (e.key == TuneKey{prec_key<R>(), 0, n, bucket_of(nsys, 0)}) vown = e.variant;
+                        if (e.key == TuneKey{prec_key<R>(), 0, n, bucket_of(nsys, 0, 1)}) vown = e.variant;
                 }
                 if (vown >= VW) vown = 0;
                 return 2 + mdot_dispatch<R>(vown, n, nullptr, 0, segB, strideB, qb, w, strideW, act, nsys, partials,
@@ -4540,7 +4594,7 @@ int mdot_dispatch(int v, int n, const typename CT<R>::t *segA, int qa, const typ
             {
                 std::lock_guard<std::mutex> lk(g_tune_mu);
                 for (auto &e : g_tuned)
-                    if (e.key == TuneKey{prec_key<R>(), 0, n, bucket_of(nsys, 0)}) vown = e.variant;
+                    if (e.key == TuneKey{prec_key<R>(), 0, n, bucket_of(nsys, 0, 1)}) vown = e.variant;
             }
             if (vown >= VW) vown = 0;
             return 2 + mdot_dispatch<R>(vown, n, nullptr, 0, segB, strideB, qb, w, strideW, act, nsys, partials, qmax,
@@ -4647,11 +4701,11 @@ void launch_mdot(int n, const typename CT<R>::t *segA, int qa, const typename CT
     };
     int v = 0;
     if (forced_variant(0) >= 0) v = forced_variant(0);
-    else if (representative(nsys, qa, qb) && !profile_enabled()) v = tuned_variant(prec_key<R>(), 0, n, nsys, qa, sizeof(R) == 4 ? 11 : 14, st, run);
+    else if (representative(nsys, qa, qb) && !profile_enabled()) v = tuned_variant(prec_key<R>(), 0, n, nsys, qa, qb, sizeof(R) == 4 ? 11 : 14, st, run);
     else {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         for (auto &e : g_tuned)
-            if (e.key == TuneKey{prec_key<R>(), 0, n, bucket_of(nsys, qa)}) v = e.variant;
+            if (e.key == TuneKey{prec_key<R>(), 0, n, bucket_of(nsys, qa, qb)}) v = e.variant;
     }
     run(v);
     L_.add(launched);
@@ -4696,7 +4750,7 @@ int update_dispatch(int v, int n, const typename CT<R>::t *segA, int qa, const t
                 {
                     std::lock_guard<std::mutex> lk(g_tune_mu);
                     for (auto &e : g_tuned)
-                        if (e.key == TuneKey{prec_key<R>(), 1, n, bucket_of(nsys, 0)}) vown = e.variant;
+                        if (e.key == TuneKey{prec_key<R>(), 1, n, bucket_of(nsys, 0, 1)}) vown = e.variant;
                 }
                 if (vown >= VW) vown = 0;
                 return 1 + update_dispatch<R>(vown, n, nullptr, 0, segB, strideB, qb + 1, w, strideW, out, strideO,
@@ -4817,14 +4871,40 @@ void launch_update(int n, const typename CT<R>::t *segA, int qa, const typename 
     int v = 0;
     if (forced_variant(1) >= 0) v = forced_variant(1);
     else if (representative(nsys, qa, qb) && !profile_enabled())
-        v = tuned_variant(prec_key<R>(), 1, n, nsys, qa, sizeof(R) == 4 ? 12 : 13, st, run);
+        v = tuned_variant(prec_key<R>(), 1, n, nsys, qa, qb, sizeof(R) == 4 ? 12 : 13, st, run);
     else {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         for (auto &e : g_tuned)
-            if (e.key == TuneKey{prec_key<R>(), 1, n, bucket_of(nsys, qa)}) v = e.variant;
+            if (e.key == TuneKey{prec_key<R>(), 1, n, bucket_of(nsys, qa, qb)}) v = e.variant;
     }
     run(v);
     L_.add(launched);
+}
+
+void launch_wdeflate(int n, int kk, const float2 *W, const float2 *y, size_t strideY, float2 *out, size_t strideO,
+                     const int *act, int nsys, double2 *coef, size_t strideC, double2 *partials, int qmax,
+                     unsigned *tickets, SysState *state, cudaStream_t st) {
+    launch_mdot<float>(n, W, kk, nullptr, 0, 0, y, strideY, act, nsys, partials, qmax, tickets, coef, strideC, state,
+                       false, st);
+    Launch L_(KC_UPDATE, (double)sizeof(float2) * n * ((double)kk + 2.0 * nsys), st, 1);
+    // 0: the tensor cores; 1-3: the update kernels (grouped over 4 or 2 systems, one system a CTA)
+    const bool tc = wapply_tc_ok(n, kk, nsys);
+    static const int update_variant[4] = {1, 6, 7, 1};
+    auto run = [&](int v) {
+        if (v == 0 && tc)
+            launch_wapply_sub_tc(n, kk, W, coef, strideC, act, nsys, y, strideY, out, strideO, st);
+        else
+            update_dispatch<float>(update_variant[v], n, W, kk, nullptr, 0, 0, y, strideY, out, strideO, act, nsys,
+                                   coef, strideC, partials, tickets, state, FinishArgs{}, false, st);
+    };
+    int v = 0;
+    if (nsys > 1 && !profile_enabled()) v = tuned_variant(prec_key<float>(), 2, n, nsys, kk, 0, 4, st, run);
+    else {
+        std::lock_guard<std::mutex> lk(g_tune_mu);
+        for (auto &e : g_tuned)
+            if (e.key == TuneKey{prec_key<float>(), 2, n, bucket_of(nsys, kk, 0)}) v = e.variant;
+    }
+    run(v);
 }
 
 template <class R>
@@ -5057,6 +5137,15 @@ SellPattern sell_pattern(const SellMatrix &A) {
     return p;
 }
 
+namespace {
+// f(OpMode constant) for a launch with these arguments (see launch_spmm)
+template <class F> void op_mode_dispatch(const SysState *scale, const void *vout, F &&f) {
+    if (!scale) f(std::integral_constant<int, OP_PLAIN>{});
+    else if (vout) f(std::integral_constant<int, OP_SCALE>{});
+    else f(std::integral_constant<int, OP_SHIFT>{});
+}
+}  // namespace
+
 template <class R>
 void launch_spmm(const SellMatrix &A, const typename CT<R>::t *x, size_t strideX, typename CT<R>::t *y, size_t strideY,
                  const int *act, int nsys, cudaStream_t st, const SysState *scale, typename CT<R>::t *vout,
@@ -5064,7 +5153,9 @@ void launch_spmm(const SellMatrix &A, const typename CT<R>::t *x, size_t strideX
     if (nsys <= 0) return;
     // with the normalisation folded in, the kernel also writes v_s: one more vector a system
     Launch L_(KC_SPMM, spmm_bytes(A, sizeof(typename CT<R>::t), nsys) +
-                           (scale ? (double)sizeof(typename CT<R>::t) * A.n * nsys : 0.0), st, 1);
+                           (vout ? (double)sizeof(typename CT<R>::t) * A.n * nsys : 0.0), st, 1);
+    op_mode_dispatch(scale, vout, [&](auto mode) {
+    constexpr int MODE = decltype(mode)::value;
     const int sg = nsys == 1 ? 1 : grid_batch();
     if (A.grid && grid_operator() && sg > 0) {
         const int ntiles = ((A.gx + 31) / 32) * ((A.gy + 7) / 8), nzc = (A.gz + GR_ZC - 1) / GR_ZC;
@@ -5073,7 +5164,7 @@ void launch_spmm(const SellMatrix &A, const typename CT<R>::t *x, size_t strideX
         if (blocks <= 0x7fffffffL) {
             const auto *cf = (const typename CT<R>::t *)A.grid;
 #define GRID_LAUNCH_(SGV)                                                                                              \
-    k_grid_spmm<R, SGV><<<(unsigned)blocks, NT, 0, st>>>(A.gx, A.gy, A.gz, ngroups, ntiles, A.greal, cf, x, strideX, y, \
+    k_grid_spmm<R, SGV, MODE><<<(unsigned)blocks, NT, 0, st>>>(A.gx, A.gy, A.gz, ngroups, ntiles, A.greal, cf, x, strideX, y, \
                                                          strideY, act, nsys, scale, vout, strideVO)
             if (sg == 1)
                 GRID_LAUNCH_(1);
@@ -5087,7 +5178,7 @@ void launch_spmm(const SellMatrix &A, const typename CT<R>::t *x, size_t strideX
     }
     if (nsys == 1) {
         const long chunks = ((long)A.n + 2 * NT - 1) / (2 * NT);
-        k_spmv2<R><<<(unsigned)chunks, NT, 0, st>>>(A.n, A.slice_ptr, A.cols, (const typename CT<R>::t *)A.vals, x,
+        k_spmv2<R, MODE><<<(unsigned)chunks, NT, 0, st>>>(A.n, A.slice_ptr, A.cols, (const typename CT<R>::t *)A.vals, x,
                                                     strideX, y, strideY, act, sell_pattern(A), scale, vout,
                                                     strideVO);
         return;
@@ -5095,8 +5186,9 @@ void launch_spmm(const SellMatrix &A, const typename CT<R>::t *x, size_t strideX
     constexpr int SG = 8;
     int rows = (A.n + NT - 1) / NT;
     dim3 grid((nsys + SG - 1) / SG, rows < 65535 ? rows : 65535);
-    k_spmm<R, SG><<<grid, NT, 0, st>>>(A.n, A.slice_ptr, A.cols, (const typename CT<R>::t *)A.vals, x, strideX, y,
-                                       strideY, act, nsys, sell_pattern(A), scale, vout, strideVO);
+    k_spmm<R, SG><<<grid, NT, 0, st>>>(A.n, A.slice_ptr, A.cols, (const typename CT<R>::t *)A.vals, x, strideX,
+                                             y, strideY, act, nsys, sell_pattern(A), scale, vout, strideVO);
+    });
 }
 
 template <class R>
@@ -5106,11 +5198,15 @@ void launch_stencil(const Stencil7 &S, const typename CT<R>::t *x, size_t stride
     if (nsys <= 0) return;
     const double n = (double)S.nx * S.ny * S.nz;
     // x read once, y written (and v = a x written with the normalisation folded in)
-    Launch L_(KC_SPMM, (scale ? 3.0 : 2.0) * nsys * n * sizeof(typename CT<R>::t), st, 1);
+    Launch L_(KC_SPMM, (vout ? 3.0 : 2.0) * nsys * n * sizeof(typename CT<R>::t), st, 1);
     const int tiles = ((S.nx + 31) / 32) * ((S.ny + 7) / 8);
     const dim3 grid(tiles, (S.nz + ST_ZC - 1) / ST_ZC, nsys);
-    k_stencil<R><<<grid, NT, 0, st>>>(S.nx, S.ny, S.nz, S.d, S.wx, S.wy, S.wz, x, strideX, y, strideY, act, scale,
-                                      vout, strideVO);
+    op_mode_dispatch(scale, vout, [&](auto mode) {
+        using C = typename CT<R>::t;
+        k_stencil<R, decltype(mode)::value><<<grid, NT, 0, st>>>(
+            S.nx, S.ny, S.nz, host_value<C>(S.d), host_value<C>(S.wx), host_value<C>(S.wy), host_value<C>(S.wz), x,
+            strideX, y, strideY, act, scale, vout, strideVO);
+    });
 }
 
 int resid_pattern(const SellMatrix &A, ResidPattern &rp) {

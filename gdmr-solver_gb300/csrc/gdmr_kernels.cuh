@@ -93,7 +93,10 @@ struct SysState {
     double true_res;    // last FP64 ||b - A x|| (refined form)
     int broken;         // Krylov step at which breakdown happened this cycle (0 = none)
     int bad;            // non-finite value met
-    int pad[2];
+    int ill;            // the blocked Krylov steps gave this cycle up (gdmr_block.cu)
+    float bs_sigma;     // blocked steps: scale and shift of the next block's operator products,
+    float bs_tr, bs_ti; // y = sigma (A x - t x), t = bs_tr + i bs_ti,
+    double bs_sumr, bs_sumi;   // and the sum of the Krylov diagonal of H that t is the mean of
 };
 
 // Finishing actions run by the last CTA of a reduction kernel.
@@ -186,6 +189,21 @@ enum KernelClass : int {
     KC_COUNT = 9
 };
 long long launch_count();
+// Counts nlaunch kernels and, with profiling on, brackets them with events (the launchers of the
+// other translation units).
+class ProfScope {
+  public:
+    ProfScope(int kc, double bytes, cudaStream_t st, int nlaunch);
+    ~ProfScope();
+    ProfScope(const ProfScope &) = delete;
+    ProfScope &operator=(const ProfScope &) = delete;
+
+  private:
+    void *impl_ = nullptr;
+};
+// SMs of the current device; dynamic shared memory above 48 KB for a kernel on it (once per kernel).
+int device_sm_count();
+void block_allow_smem(const void *kernel, size_t bytes);
 void profile_enable(bool on);
 bool profile_enabled();
 void profile_flush();
@@ -209,6 +227,7 @@ std::string tune_report();
 size_t scratch_doubles(int qmax, int nsys, int n);
 // Reduction scratch handed to the Gram-Schmidt launchers must be registered with its size.
 void register_scratch(const void *p, size_t doubles);
+size_t scratch_size(const void *p);   // doubles registered for p (0: none)
 void unregister_scratch(const void *p);
 
 template <class R>
@@ -239,6 +258,9 @@ int launch_wproj_tc(int n, int kk, const float2 *W, const float2 *Y, size_t stri
 bool wapply_tc_ok(int n, int kk, int nsys);
 int launch_wapply_tc(int n, int kk, const float2 *W, double2 *coef, size_t strideC, const int *act, int nsys,
                      float2 *P, size_t strideP, int unit_idx, cudaStream_t st);
+// The same product subtracted: out_s = y_s - W c_s (out and y distinct).
+int launch_wapply_sub_tc(int n, int kk, const float2 *W, const double2 *coef, size_t strideC, const int *act, int nsys,
+                         const float2 *y, size_t strideY, float2 *out, size_t strideO, cudaStream_t st);
 // The batched update with its shared part on the tensor cores in one kernel (complex64;
 // gdmr_tc.cu): out_s = w_s - V_s c_s[kk..kk+qb) - W c_s[0..kk) for the active systems, with
 // ||out_s||^2 and <out_s, w_s> reduced through partials (wupdate_tc_grid(n) x 3 x nsys doubles)
@@ -250,6 +272,23 @@ int launch_wupdate_tc(int n, int kk, const float2 *W, const float2 *V, size_t st
                       size_t strideW, float2 *out, size_t strideO, const int *act, int nsys, const double2 *coef,
                       size_t strideC, double *partials, unsigned *tickets, SysState *state, FinishArgs fin,
                       bool skip_broken, cudaStream_t st);
+// out_s = y_s - W W^H y_s for the active systems (complex64), a_s = W^H y_s into coef (out and y
+// distinct): the deflator of a blocked Krylov step.
+void launch_wdeflate(int n, int kk, const float2 *W, const float2 *y, size_t strideY, float2 *out, size_t strideO,
+                     const int *act, int nsys, double2 *coef, size_t strideC, double2 *partials, int qmax,
+                     unsigned *tickets, SysState *state, cudaStream_t st);
+// Blocked Krylov steps (gdmr_block.cu): KRYLOV_BLOCK steps sharing their passes over the own basis.
+constexpr int KRYLOV_BLOCK = 3;
+size_t krylov_block_scratch(int m, int nsys);
+bool krylov_block_fits(int m, int n, int nsys, size_t capacity);
+// Shift and scale of the first block, from the first `cols` Krylov columns of H.
+void launch_block_init(int cols, int kk, int m, const int *act, int nsys, SysState *state, const double2 *H,
+                       size_t strideH, cudaStream_t st);
+// One block: basis slots nv .. nv + 2 hold y_1 .. y_3 and become the next three basis vectors; H gets
+// its columns kk + nv - 1 .. kk + nv + 1.  a[b]: W^H of the b-th operator product (unused when kk = 0).
+void launch_block_step(int n, int nv, int kk, int m, float2 *V, size_t strideV, const int *act, int nsys,
+                       SysState *state, double2 *H, size_t strideH, const double2 *const (&a)[KRYLOV_BLOCK],
+                       size_t strideC, double tol, double *scratch, size_t capacity, cudaStream_t st);
 // mbarrier waits of the tensor-core kernels that ran out of time (0 in a healthy process).
 unsigned wproj_tc_timeouts();
 // Bounded mbarrier waits of the bulk-copy Gram-Schmidt pipelines and grid barriers of the fused
@@ -359,12 +398,14 @@ struct Stencil7 {
     int nx, ny, nz;
     double2 d, wx, wy, wz;
 };
-// `scale` / vout: the pending normalisation, as for launch_spmm.
+// `scale` / vout: the pending normalisation or the shifted product, as for launch_spmm.
 template <class R>
 void launch_stencil(const Stencil7 &S, const typename CT<R>::t *x, size_t strideX, typename CT<R>::t *y,
                     size_t strideY, const int *act, int nsys, cudaStream_t st, const SysState *scale = nullptr,
                     typename CT<R>::t *vout = nullptr, size_t strideVO = 0);
 
+// With `scale` and a null vout: y_s = sigma_s (A x_s - t_s x_s), the shifted product of the blocked
+// Krylov steps (scale[s].bs_*).
 // With `scale` (the pending normalisation): x holds the unnormalised Krylov vectors w_s, y_s =
 // a_s (A w_s) and v_s = a_s w_s (zero after a breakdown) is written to vout (a_s = scale[s].alpha).
 template <class R>

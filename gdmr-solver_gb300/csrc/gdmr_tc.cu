@@ -452,10 +452,13 @@ __device__ __forceinline__ int swz(int r, int kf, int rows) {   // float offset 
     return ((kf >> 5) * rows * TC_ROW + r * TC_ROW + ((((kf >> 2) & 7) ^ (r & 7)) << 4) + ((kf & 3) << 2)) >> 2;
 }
 
+// SUB: out_s = y_s - W c_s instead (the deflator of a blocked Krylov step; no unit coefficient).  A
+// group's eight y values are loaded before its TMEM reads, so they are in flight together.
+template <bool SUB>
 __global__ void __launch_bounds__(WA_THREADS, 1)
     k_wapply_tc(int n, int kk, const float2 *__restrict__ W, double2 *__restrict__ coef0, size_t strideC,
                 const int *__restrict__ act, int nsys, int nsp, float2 *__restrict__ P0, size_t strideP,
-                int unit_idx) {
+                int unit_idx, const float2 *__restrict__ Y0, size_t strideY) {
     extern __shared__ __align__(1024) unsigned char wa_sm[];
     unsigned char *base = wa_sm + ((1024u - (smem_u32(wa_sm) & 1023u)) & 1023u);
     float *A = reinterpret_cast<float *>(base);                       // [buf][big|small] operands
@@ -503,7 +506,8 @@ __global__ void __launch_bounds__(WA_THREADS, 1)
                 B[swz(2 * nsp + 2 * sl + o, 2 * p + q, brows)] = v - big;
             }
     }
-    if (blockIdx.x == 0 && tid < nsys) coef0[(size_t)s_act[tid] * strideC + unit_idx] = make_double2(1.0, 0.0);
+    if (!SUB && blockIdx.x == 0 && tid < nsys)
+        coef0[(size_t)s_act[tid] * strideC + unit_idx] = make_double2(1.0, 0.0);
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
@@ -603,6 +607,14 @@ __global__ void __launch_bounds__(WA_THREADS, 1)
             const long g = ((long)blockIdx.x + (long)i * G) * WA_TILE + quarter * 32 + lane;
             const uint32_t row = taddr + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * 256);
             for (int c0 = 16 * part; c0 < 2 * nsp; c0 += 16 * (WA_EPI / 4)) {
+                float2 y[8];
+                if constexpr (SUB) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const int sl = c0 / 2 + j;
+                        y[j] = (g < n && sl < nsys) ? Y0[(size_t)s_act[sl] * strideY + g] : make_float2(0.f, 0.f);
+                    }
+                }
                 uint32_t vb[16], vs[16];
                 tmem_ld16(row + (uint32_t)c0, vb);
                 tmem_ld16(row + (uint32_t)(2 * nsp + c0), vs);
@@ -610,10 +622,11 @@ __global__ void __launch_bounds__(WA_THREADS, 1)
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
                         const int sl = c0 / 2 + j;
+                        const float pr = __uint_as_float(vb[2 * j]) + __uint_as_float(vs[2 * j]),
+                                    pi = __uint_as_float(vb[2 * j + 1]) + __uint_as_float(vs[2 * j + 1]);
                         if (sl < nsys)
-                            P0[(size_t)s_act[sl] * strideP + g] =
-                                make_float2(__uint_as_float(vb[2 * j]) + __uint_as_float(vs[2 * j]),
-                                            __uint_as_float(vb[2 * j + 1]) + __uint_as_float(vs[2 * j + 1]));
+                            P0[(size_t)s_act[sl] * strideP + g] = SUB ? make_float2(y[j].x - pr, y[j].y - pi)
+                                                                      : make_float2(pr, pi);
                     }
                 }
             }
@@ -963,8 +976,10 @@ size_t wapply_smem_bytes(int nsp) { return (size_t)4 * WA_AOP + (size_t)4 * nsp 
 
 bool wapply_tc_ok(int n, int kk, int nsys) { return kk > 0 && kk <= TC_KMAX && nsys >= 8 && nsys <= TC_NMAX && n > 0; }
 
-int launch_wapply_tc(int n, int kk, const float2 *W, double2 *coef, size_t strideC, const int *act, int nsys,
-                     float2 *P, size_t strideP, int unit_idx, cudaStream_t st) {
+namespace {
+template <bool SUB>
+int wapply_run(int n, int kk, const float2 *W, double2 *coef, size_t strideC, const int *act, int nsys, float2 *P,
+               size_t strideP, int unit_idx, const float2 *y, size_t strideY, cudaStream_t st) {
     int dev = 0;
     cudaGetDevice(&dev);
     const long ntiles = ((long)n + WA_TILE - 1) / WA_TILE;
@@ -976,14 +991,25 @@ int launch_wapply_tc(int n, int kk, const float2 *W, double2 *coef, size_t strid
         std::lock_guard<std::mutex> lk(g_tc_mu);
         if ((int)set.size() <= dev) set.resize(dev + 1, 0);
         if (!set[dev]) {
-            cudaFuncSetAttribute(k_wapply_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            cudaFuncSetAttribute(k_wapply_tc<SUB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)wapply_smem_bytes(TC_NMAX));
             set[dev] = 1;
         }
     }
-    k_wapply_tc<<<G, WA_THREADS, wapply_smem_bytes(nsp), st>>>(n, kk, W, coef, strideC, act, nsys, nsp, P, strideP,
-                                                               unit_idx);
+    k_wapply_tc<SUB><<<G, WA_THREADS, wapply_smem_bytes(nsp), st>>>(n, kk, W, coef, strideC, act, nsys, nsp, P, strideP,
+                                                                    unit_idx, y, strideY);
     return 1;
+}
+}  // namespace
+
+int launch_wapply_tc(int n, int kk, const float2 *W, double2 *coef, size_t strideC, const int *act, int nsys,
+                     float2 *P, size_t strideP, int unit_idx, cudaStream_t st) {
+    return wapply_run<false>(n, kk, W, coef, strideC, act, nsys, P, strideP, unit_idx, nullptr, 0, st);
+}
+
+int launch_wapply_sub_tc(int n, int kk, const float2 *W, const double2 *coef, size_t strideC, const int *act, int nsys,
+                         const float2 *y, size_t strideY, float2 *out, size_t strideO, cudaStream_t st) {
+    return wapply_run<true>(n, kk, W, const_cast<double2 *>(coef), strideC, act, nsys, out, strideO, -1, y, strideY, st);
 }
 
 size_t wupdate_smem_bytes(int nsp) {
