@@ -336,6 +336,27 @@ int sell_from_csr(DeviceSell &out, int n, const int *rowptr, const int *colidx, 
             for (int r = 0; real && r < n; ++r) real = gim[(size_t)e * n + r] == 0.0;
             if (real) d.greal |= 1u << e;
         }
+        // constant planes: one value wherever the neighbour lies on the grid
+        bool same = true;
+        const long plane = (long)gx * gy;
+        const int p0 = gz > 1 ? 0 : 1;
+        for (int e = 0; same && e < np; ++e) {
+            const int p = e + p0;                       // 7-plane index: -P, -Q, -1, 0, +1, +Q, +P
+            bool any = false;
+            double re = 0, im = 0;
+            for (int r = 0; same && r < n; ++r) {
+                const int x = r % gx, y = (int)((r / gx) % gy), z = (int)(r / plane);
+                if ((p == 0 && z == 0) || (p == 1 && y == 0) || (p == 2 && x == 0) || (p == 4 && x + 1 == gx) ||
+                    (p == 5 && y + 1 == gy) || (p == 6 && z + 1 == gz))
+                    continue;
+                const double a = gre[(size_t)e * n + r], b = gim[(size_t)e * n + r];
+                if (!any) { re = a; im = b; any = true; }
+                same = a == re && b == im;
+            }
+            d.gconst.a[p] = make_double2(re, im);
+            if (im == 0.0) d.gconst.real |= 1u << p;
+        }
+        d.gconst.valid = same;
         // one precision at a time, each host copy released after its upload
         if (want32) {
             std::vector<float2> g(gsz);

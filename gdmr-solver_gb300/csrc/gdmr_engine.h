@@ -50,6 +50,7 @@ struct DeviceSell {
     dfc *griddf = nullptr;
     int gx = 0, gy = 0, gz = 0;
     unsigned greal = 0;                // bit p: plane p is real (imaginary parts all zero)
+    GridConst gconst;                  // the planes' values, if every plane is constant
     unsigned preal = 0;                // bit e: entry e of every pattern-stored slice is real
     SellMatrix view(const void *v, const void *g) const {
         SellMatrix m{n, nslices, slice_ptr, cols, v, nnz};
@@ -62,6 +63,7 @@ struct DeviceSell {
         m.gz = gz;
         m.greal = greal;
         m.preal = preal;
+        m.gconst = gconst;
         return m;
     }
     SellMatrix view32() const { return view(vals32, grid32); }

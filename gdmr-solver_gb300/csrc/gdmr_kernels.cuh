@@ -365,6 +365,13 @@ struct SellPattern {
     const unsigned char *uniform;
     int off[SELL_PATTERN];
 };
+// A grid form whose planes are constant: every row that has a neighbour on the grid in the plane's
+// direction holds the same value there.  Values in the 7-plane order (2D: the middle five).
+struct GridConst {
+    double2 a[7];
+    unsigned real = 0;    // bit p: a[p] has a zero imaginary part
+    bool valid = false;
+};
 struct SellMatrix {
     int n;              // rows
     int nslices;        // ceil(n/32)
@@ -382,6 +389,7 @@ struct SellMatrix {
     int gx = 0, gy = 0, gz = 0;
     unsigned greal = 0;   // bit p: every value of plane p has a zero imaginary part
     unsigned preal = 0;   // bit e: entry e of every pattern-stored slice has a zero imaginary part
+    GridConst gconst;
 };
 // Process-wide switch for the structured-grid operator kernel (on by default); launch_spmm
 // takes the SELL kernels when it is off or the matrix has no grid form.  grid_batch: systems a

@@ -168,7 +168,8 @@ void gdmrTuneForce(int projectionVariant, int updateVariant);
 void gdmrGridOperator(int enable);
 /* Products over several systems at once (the batched solves) take the grid kernel only when
  * this is 1, 2 or 4 (systems a thread; the coefficients are loaded once for them); 0, the
- * default, keeps them on the SELL-32 kernel, which measured faster for the 64-system batch. */
+ * default, keeps them on the SELL-32 kernel, which measured faster for the 64-system batch, or, when
+ * every coefficient plane is constant, on a kernel that reads no coefficients (0 at any batch size). */
 void gdmrGridBatch(int systemsPerThread);
 
 /* The cycle-end combinations (r -= [W V] t, x += rho [Z V] y) of batches of four or more

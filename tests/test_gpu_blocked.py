@@ -1,4 +1,4 @@
-"""Blocked Krylov steps of the refined complex64 batches (gdmr_block.cu).
+"""Blocked Krylov steps of the refined complex64 batches (gdmr_block.cu) and the constant-plane operator.
 
 The blocked loop runs when n x systems reaches 3 * 2^17; every shape here is just above that."""
 import numpy as np
@@ -78,3 +78,31 @@ def test_exhausted_krylov_space_falls_back(eigenvalues):
         X, stats = s.solve_batch(B, tol=TOL, max_cycles=60)
         _check(A, B, X, stats)
     s.close()
+
+
+@pytest.mark.parametrize("shape,nrhs,factor,precision", [
+    ((41, 39, 33), 8, 1.0, "mixed"),            # real off-diagonal planes, partial tiles, shifted products
+    ((41, 39, 33), 8, 0.6 + 0.8j, "mixed"),     # complex planes
+    ((67, 45), 3, 1.0, "mixed"),                # 2D, step by step
+    ((20, 12, 19), 1, 1.0, "fp64"),
+    ((20, 12, 19), 2, 0.6 + 0.8j, "fp64e"),
+])
+def test_constant_plane_operator_matches_sell(shape, nrhs, factor, precision):
+    # the terms and their order are the SELL kernel's, so whole solves agree bit for bit
+    A = _scaled(problems.helmholtz(shape, 5.0, 0.1), factor)
+    B = _rhs(A.n, nrhs)
+    out = []
+    for grid in (True, False):
+        gdmr.grid_operator(grid)
+        try:
+            s = gdmr.System(A, 30, 8, capacity=nrhs, precision=precision)
+            s.set_fused(False)
+            s.solve_batch(B, tol=TOL, max_cycles=400)      # every launch's kernel variant settled
+            s.drop_deflation()
+            X, stats = s.solve_batch(B, tol=TOL, max_cycles=400)
+            s.close()
+        finally:
+            gdmr.grid_operator(True)
+        _check(A, B, X, stats)
+        out.append(X)
+    assert np.array_equal(out[0], out[1])
