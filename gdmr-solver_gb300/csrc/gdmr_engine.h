@@ -260,7 +260,7 @@ template <class R> class Engine {
     struct GraphEntry {
         int kk, nsys, zpar;
         double tol;
-        bool blocked;
+        bool blocked, cholqr;
         cudaGraphExec_t exec;
     };
     std::vector<GraphEntry> graphs_;
@@ -273,6 +273,11 @@ template <class R> class Engine {
     // Blocked Krylov steps: blocked_ is set around a refined complex64 cycle while blocks_on_ (from
     // refine_setup until a system's block turns out ill-conditioned).
     bool blocked_ = false, blocks_on_ = true;
+    // Cholesky QR in the deflation loop: refined_ is set around refined cycles, cholqr_on_ until a factor
+    // breaks down.
+    bool refined_ = false, cholqr_on_ = true;
+    bool cholqr_ok(int kk) const;
+    void enqueue_deflation_cholqr(int kk, long *matvecs);
     bool blocked_ok(int kk, int nsys) const;
     int enqueue_krylov_blocked(int kk, int nsys, double tol, long *matvecs);
     // lockstep (many-operator) form: the cycle the last multi_front set up

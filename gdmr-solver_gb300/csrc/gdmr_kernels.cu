@@ -4055,11 +4055,12 @@ __global__ void __launch_bounds__(NT) k_copy(int n, const typename CT<R>::t *__r
 template <class R>
 __global__ void __launch_bounds__(NT) k_refine_update(int n, double2 *__restrict__ x0, size_t strideX,
                                                       typename CT<R>::t *__restrict__ d0, size_t strideD,
-                                                      const int *__restrict__ act, const SysState *__restrict__ state) {
+                                                      const int *__restrict__ act, const SysState *__restrict__ state,
+                                                      int shared) {
     using C = typename CT<R>::t;
     const int s = act[blockIdx.y];
     const double sc = state[s].true_res;
-    const bool drop = state[s].ill != 0;   // the cycle's correction is not used
+    const bool drop = state[s].ill != 0 || state[shared].ill != 0;   // the cycle's correction is not used
     double2 *x = x0 + (size_t)s * strideX;
     C *d = d0 + (size_t)s * strideD;
     for (long i = (long)blockIdx.x * NT + threadIdx.x; i < n; i += (long)gridDim.x * NT) {
@@ -4138,6 +4139,92 @@ __global__ void __launch_bounds__(NT) k_norm(int n, const typename CT<R>::t *__r
         if (mode == 2) { st.rho_abs = nr; st.alpha = nr > 0 ? 1.0 / nr : 0.0; }
         if (!isfinite(nr)) st.bad = 1;
         tickets[slot] = 0;
+    }
+}
+
+// See launch_cholqr.  One CTA, thread (x, y) = entry (row y, column x); right-looking, in double-float
+// (a native FP64 update of the trailing block is ~2500 clocks a column on GB300).  Latency-bound.
+__global__ void __launch_bounds__(1024) k_cholqr(int k, double2 *__restrict__ gram, int ldg, double2 *__restrict__ rout,
+                                                 const double2 *__restrict__ r1, double2 *__restrict__ hd, int ldh,
+                                                 SysState *st) {
+    constexpr int K = CHOLQR_MAX;
+    __shared__ dfc S[K][K + 1], E[K][K + 1];   // S: G, then R; E: the inverse of R^H
+    __shared__ float dmax, diag[K];
+    __shared__ int s_bad;
+    const int x = threadIdx.x, y = threadIdx.y, tid = y * K + x;
+    if (tid == 0) s_bad = 0;
+    if (y == 0) {
+        float d = x < k ? (float)gram[(size_t)x * ldg + x].x : 0.f;
+        for (int o = 16; o > 0; o >>= 1) d = fmaxf(d, __shfl_xor_sync(0xffffffffu, d, o));
+        if (x == 0) dmax = d;
+    }
+    __syncthreads();
+    // scaled by an even power of two, so that nothing leaves the FP32 range and R scales exactly
+    const int ex = (dmax > 0.f && dmax < 3e38f) ? (ilogbf(dmax) & ~1) : 0;
+    if (x < k && y < k) {
+        const double2 g = gram[(size_t)x * ldg + y];
+        dfc c;
+        c.x = dfr(ldexp(g.x, -ex));
+        c.y = dfr(x == y ? 0.0 : ldexp(g.y, -ex));
+        S[y][x] = c;
+        if (x == y) diag[x] = c.x.hi;
+        c.x = dfr(x == y ? 1.f : 0.f, 0.f);
+        c.y = dfr(0.f, 0.f);
+        E[y][x] = c;
+    }
+    __syncthreads();
+    for (int j = 0; j < k; ++j) {
+        const dfr piv = S[j][j].x;
+        const bool ok = piv.hi > 1e-3f * diag[j] && piv.hi < 3e38f;   // false for NaN
+        if (!ok) {
+            if (tid == 0) s_bad = 1;
+            break;                                   // uniform: every thread reads the same pivot
+        }
+        const dfr inv = df_rsqrt(piv);
+        __syncthreads();
+        if (y == j && x < k) {
+            dfc &s = S[j][x], &e = E[j][x];
+            if (x >= j) { s.x = s.x * inv; s.y = s.y * inv; }
+            if (x <= j) { e.x = e.x * inv; e.y = e.y * inv; }
+        }
+        __syncthreads();
+        if (y > j && y < k && x < k) {
+            const dfc l = S[j][y];                   // conj(R[j][y]) times row j
+            dfc *t = x >= y ? &S[y][x] : nullptr;
+            if (t) {
+                const dfc r = S[j][x];
+                t->x = t->x - (l.x * r.x + l.y * r.y);
+                t->y = t->y - (l.x * r.y - l.y * r.x);
+            }
+            if (x <= j) {
+                const dfc r = E[j][x];
+                E[y][x].x = E[y][x].x - (l.x * r.x + l.y * r.y);
+                E[y][x].y = E[y][x].y - (l.x * r.y - l.y * r.x);
+            }
+        }
+        __syncthreads();
+    }
+    __syncthreads();
+    const bool bad = s_bad != 0;
+    if (tid == 0 && (bad || !r1)) st->ill = bad ? 2 : 0;
+    if (x >= k || y >= k) return;
+    const int hx = ex / 2;
+    const double2 zero = make_double2(0.0, 0.0);
+    // R[y][x] and R^-1[y][x] = conj(E[x][y])
+    const double2 r = (bad || y > x) ? zero
+                                     : make_double2(ldexp((double)S[y][x].x, hx), ldexp((double)S[y][x].y, hx));
+    rout[(size_t)x * k + y] = r;
+    gram[(size_t)x * ldg + y] =
+        (bad || y > x) ? zero : make_double2(ldexp((double)E[x][y].x, -hx), -ldexp((double)E[x][y].y, -hx));
+    if (r1) {
+        double2 h = zero;
+        if (!bad)
+            for (int l = y; l <= x; ++l) {
+                const double2 a = make_double2((double)S[y][l].x, (double)S[y][l].y), b = r1[(size_t)x * k + l];
+                h.x += a.x * b.x - a.y * b.y;
+                h.y += a.x * b.y + a.y * b.x;
+            }
+        hd[(size_t)x * ldh + y] = y > x ? zero : make_double2(ldexp(h.x, hx), ldexp(h.y, hx));
     }
 }
 
@@ -4393,8 +4480,9 @@ thread_local bool t_capturing = false;   // a stream capture is open on this thr
 // Engines run their first two cycles eagerly, so every class they use is settled before a
 // cycle is captured into a CUDA graph.
 int bucket_of(int nsys, int qa, int qb) {
-    // a batch against the shared vectors alone (the deflator of the blocked Krylov steps) is its own class
-    return (nsys > 1 ? 1 : 0) + (qa > 0 ? 2 : 0) + (nsys > 1 && qa > 0 && qb == 0 ? 4 : 0);
+    // a batch against the shared vectors alone (the deflator of the blocked Krylov steps, the deflation
+    // loop's Gram matrix) is its own class, in two for the batches that can and cannot take the tensor cores
+    return (nsys > 1 ? 1 : 0) + (qa > 0 ? 2 : 0) + (nsys > 1 && qa > 0 && qb == 0 ? (nsys >= 8 ? 12 : 4) : 0);
 }
 
 // A class is tuned on its first launch with at least 8 own-basis vectors (mid-cycle Krylov
@@ -4943,6 +5031,12 @@ void launch_update(int n, const typename CT<R>::t *segA, int qa, const typename 
     L_.add(launched);
 }
 
+void launch_cholqr(int k, double2 *gram, int ldg, double2 *r, const double2 *r1, double2 *hd, int ldh, SysState *st,
+                   cudaStream_t stream) {
+    Launch L_(KC_OTHER, 0.0, stream, 1);
+    k_cholqr<<<1, dim3(CHOLQR_MAX, CHOLQR_MAX), 0, stream>>>(k, gram, ldg, r, r1, hd, ldh, st);
+}
+
 void launch_wdeflate(int n, int kk, const float2 *W, const float2 *y, size_t strideY, float2 *out, size_t strideO,
                      const int *act, int nsys, double2 *coef, size_t strideC, double2 *partials, int qmax,
                      unsigned *tickets, SysState *state, cudaStream_t st) {
@@ -5332,10 +5426,10 @@ void launch_copy_vec(int n, const typename CT<R>::t *src, size_t strideS, typena
 
 template <class R>
 void launch_refine_update(int n, double2 *x, size_t strideX, typename CT<R>::t *d, size_t strideD, const int *act,
-                          int nsys, const SysState *state, cudaStream_t st) {
+                          int nsys, const SysState *state, int shared, cudaStream_t st) {
     if (nsys <= 0) return;
     Launch L_(KC_OTHER, (double)(sizeof(typename CT<R>::t) * 2 + sizeof(double2) * 2) * n * nsys, st, 1);
-    k_refine_update<R><<<grid2(stream_grid<R>(n, nsys), nsys), NT, 0, st>>>(n, x, strideX, d, strideD, act, state);
+    k_refine_update<R><<<grid2(stream_grid<R>(n, nsys), nsys), NT, 0, st>>>(n, x, strideX, d, strideD, act, state, shared);
 }
 
 template <class R>
@@ -5386,7 +5480,7 @@ void launch_broadcast_hdef(int m, int kk, const double2 *Hd, double2 *H, size_t 
     template void launch_copy_vec<R>(int, const CT<R>::t *, size_t, CT<R>::t *, size_t, const int *, int,              \
                                      cudaStream_t);                                                                    \
     template void launch_refine_update<R>(int, double2 *, size_t, CT<R>::t *, size_t, const int *, int,                \
-                                          const SysState *, cudaStream_t);                                             \
+                                          const SysState *, int, cudaStream_t);                                        \
     template void launch_demote_unit<R>(int, const double2 *, size_t, CT<R>::t *, size_t, CT<R>::t *, size_t,         \
                                         const int *, int, const SysState *, cudaStream_t);                             \
     template void launch_norm<R>(int, const CT<R>::t *, size_t, const int *, int, double2 *, unsigned *, SysState *,   \

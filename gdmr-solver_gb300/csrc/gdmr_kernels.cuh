@@ -93,7 +93,8 @@ struct SysState {
     double true_res;    // last FP64 ||b - A x|| (refined form)
     int broken;         // Krylov step at which breakdown happened this cycle (0 = none)
     int bad;            // non-finite value met
-    int ill;            // the blocked Krylov steps gave this cycle up (gdmr_block.cu)
+    int ill;            // the cycle's correction is dropped: 1 the blocked Krylov steps gave it up
+                        // (gdmr_block.cu); in the shared pseudo-system 2: the deflation loop's factor did
     float bs_sigma;     // blocked steps: scale and shift of the next block's operator products,
     float bs_tr, bs_ti; // y = sigma (A x - t x), t = bs_tr + i bs_ti,
     double bs_sumr, bs_sumi;   // and the sum of the Krylov diagonal of H that t is the mean of
@@ -255,7 +256,7 @@ int launch_wproj_tc(int n, int kk, const float2 *W, const float2 *Y, size_t stri
 // P[act[s]*strideP + i] = sum_p coef[act[s]*strideC + p] W_p[i] for p < kk, and
 // coef[act[s]*strideC + unit_idx] = 1, so that a per-system update with P as one more basis
 // vector subtracts W c_s.  wapply_tc_ok: kk <= 32, 8 <= nsys <= 64.
-bool wapply_tc_ok(int n, int kk, int nsys);
+bool wapply_tc_ok(int n, int kk, int nsys);   // unit_idx < 0: no unit coefficient
 int launch_wapply_tc(int n, int kk, const float2 *W, double2 *coef, size_t strideC, const int *act, int nsys,
                      float2 *P, size_t strideP, int unit_idx, cudaStream_t st);
 // The same product subtracted: out_s = y_s - W c_s (out and y distinct).
@@ -277,6 +278,15 @@ int launch_wupdate_tc(int n, int kk, const float2 *W, const float2 *V, size_t st
 void launch_wdeflate(int n, int kk, const float2 *W, const float2 *y, size_t strideY, float2 *out, size_t strideO,
                      const int *act, int nsys, double2 *coef, size_t strideC, double2 *partials, int qmax,
                      unsigned *tickets, SysState *state, cudaStream_t st);
+// One pass of the deflation loop's Cholesky QR (complex64 vectors): from the Gram matrix gram[i*ldg + l] =
+// <a_l, a_i> of k <= 32 vectors, the factor R (R^H R = G) into r (k x k, column-major) and R^-1 in
+// place of gram: column i at gram + i*ldg.  With r1, the factor of the pass before, R r1 goes to hd
+// (leading dimension ldh), the deflation block of the Hessenberg.  A pivot below 1e-3 of its column
+// makes the results zero and sets st->ill (of the shared pseudo-system) to 2; the first pass (r1 null)
+// clears it otherwise.
+constexpr int CHOLQR_MAX = 32;
+void launch_cholqr(int k, double2 *gram, int ldg, double2 *r, const double2 *r1, double2 *hd, int ldh, SysState *st,
+                   cudaStream_t stream);
 // Blocked Krylov steps (gdmr_block.cu): KRYLOV_BLOCK steps sharing their passes over the own basis.
 constexpr int KRYLOV_BLOCK = 3;
 size_t krylov_block_scratch(int m, int nsys);
@@ -540,10 +550,11 @@ void launch_dense_gemv(int n, const typename CT<R>::t *A, const typename CT<R>::
 template <class R>
 void launch_copy_vec(int n, const typename CT<R>::t *src, size_t strideS, typename CT<R>::t *dst, size_t strideD,
                      const int *act, int nsys, cudaStream_t st);
-// x64_s += scale_s * d_s (d complex64/128 inner correction), then d_s = 0.
+// x64_s += scale_s * d_s (d complex64/128 inner correction), then d_s = 0; no correction where the system
+// or the shared pseudo-system state[shared] is flagged ill.
 template <class R>
 void launch_refine_update(int n, double2 *x, size_t strideX, typename CT<R>::t *d, size_t strideD,
-                          const int *act, int nsys, const SysState *state, cudaStream_t st);
+                          const int *act, int nsys, const SysState *state, int shared, cudaStream_t st);
 // rhat_s = (R) (r64_s / sqrt(nrm2_s)); also into v0_s (the cycle's first basis vector) unless
 // v0 is null.
 template <class R>

@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(WA_THREADS, 1)
                 B[swz(2 * nsp + 2 * sl + o, 2 * p + q, brows)] = v - big;
             }
     }
-    if (!SUB && blockIdx.x == 0 && tid < nsys)
+    if (!SUB && unit_idx >= 0 && blockIdx.x == 0 && tid < nsys)
         coef0[(size_t)s_act[tid] * strideC + unit_idx] = make_double2(1.0, 0.0);
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");

@@ -80,6 +80,23 @@ def test_exhausted_krylov_space_falls_back(eigenvalues):
     s.close()
 
 
+@pytest.mark.parametrize("case", ["random", "repeated"])
+def test_imported_deflation_spaces_through_the_cholesky_factor(case):
+    # W = orth(A Z) by Cholesky QR: any independent Z works; a singular one costs
+    # the cycle and goes on step by step
+    A = problems.helmholtz((41, 39, 33), 5.0, 0.1)
+    B = _rhs(A.n, 4)
+    Z = np.stack([problems.unit_gaussian_rhs(A.n, 900 + i) for i in range(16)])
+    if case == "repeated":
+        Z[9] = Z[3]
+    s = gdmr.System(A, 40, 16, capacity=4, precision="mixed")
+    s.import_deflation(Z)
+    for _ in range(2):                   # then from the space that the first solve left
+        X, stats = s.solve_batch(B, tol=TOL, max_cycles=400)
+        _check(A, B, X, stats)
+    s.close()
+
+
 @pytest.mark.parametrize("shape,nrhs,factor,precision", [
     ((41, 39, 33), 8, 1.0, "mixed"),            # real off-diagonal planes, partial tiles, shifted products
     ((41, 39, 33), 8, 0.6 + 0.8j, "mixed"),     # complex planes
