@@ -1586,17 +1586,17 @@ __global__ void __launch_bounds__(KM_THREADS, 3) k_krylov_multi(const KrylovJob<
 }
 
 // ----------------------------------------------------------------- batched W projection
-// coef_s[p] = <W_p, y_s> for every active system s and deflation vector p: the shared part
+// coef_s[p] = <W_p, y_s> for every active system s and deflation vector p (complex128): the shared part
 // of a batched projection as one split-K product, so W is read once for the whole batch
 // instead of once per system.  Persistent CTAs walk row tiles; a tile of W (kk x RT) and of
 // the batch (nsys x RT) is copied into shared memory with cp.async, double-buffered, in its
 // natural vector-major layout (leading dimension RT+2, so the strided thread tiling below
 // reads distinct banks).  Thread (ip, js) of row group grp accumulates the 4 x 4 outputs
 // p = ip + tilesP*a, s = js + tilesS*b over the rows grp, grp+KS, ... of each tile, and
-// flushes them to double after every tile.  The KS row groups are summed in shared memory
+// converts them to double at the end.  The KS row groups are summed in shared memory
 // in a fixed order, and k_wproj_reduce sums the CTAs' partials in a fixed order.
 constexpr int WP_KMAX = 32, WP_SMAX = 64;
-template <class R> __host__ __device__ constexpr int wp_rt() { return sizeof(R) == 4 ? 64 : 32; }
+template <class R> __host__ __device__ constexpr int wp_rt() { return 32; }
 
 __device__ __forceinline__ void cp_async_el(void *dst, const void *src, int bytes, bool valid) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -1666,12 +1666,11 @@ __global__ void __launch_bounds__(NT, 2) k_wproj(int n, int kk, const typename C
         cp_async_commit();
     };
     double2 accd[4][4];
-    C acc[4][4];   // complex64: one tile's sums; complex128: the running sums
+    C acc[4][4];
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            accd[a][c] = make_double2(0.0, 0.0);
             acc[a][c] = czero<C>();
         }
     int b = 0;
@@ -1684,12 +1683,6 @@ __global__ void __launch_bounds__(NT, 2) k_wproj(int n, int kk, const typename C
         if (mine) {
             const C *Wt = buf + (size_t)b * stage;
             const C *Yt = Wt + (size_t)sh.KP * LD;
-            if constexpr (sizeof(R) == 4) {
-#pragma unroll
-                for (int a = 0; a < 4; ++a)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) acc[a][c] = czero<C>();
-            }
 #pragma unroll 2
             for (int r = grp; r < RT; r += sh.KS) {
                 C wv[4], yv[4];
@@ -1702,24 +1695,13 @@ __global__ void __launch_bounds__(NT, 2) k_wproj(int n, int kk, const typename C
 #pragma unroll
                     for (int c = 0; c < 4; ++c) cdotacc(acc[a][c], wv[a], yv[c]);
             }
-            if constexpr (sizeof(R) == 4) {   // complex64: flush the tile's sums to double
-#pragma unroll
-                for (int a = 0; a < 4; ++a)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        accd[a][c].x += (double)acc[a][c].x;
-                        accd[a][c].y += (double)acc[a][c].y;
-                    }
-            }
         }
         __syncthreads();
     }
-    if constexpr (sizeof(R) == 8) {
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < 4; ++a)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) accd[a][c] = make_double2(acc[a][c].x, acc[a][c].y);
-    }
+        for (int c = 0; c < 4; ++c) accd[a][c] = make_double2(acc[a][c].x, acc[a][c].y);
     // sum the row groups (fixed order) through shared memory, then write this CTA's partials
     double2 *red = reinterpret_cast<double2 *>(wp_sm);   // [thread][16]
     if (mine && grp > 0)
@@ -1767,6 +1749,134 @@ __global__ void __launch_bounds__(NT) k_wproj_reduce(int kk, int nsys, int G, co
     re = warp_sum(re);
     im = warp_sum(im);
     if (lane == 0) coef0[(size_t)act[sl] * strideC + p] = make_double2(re, im);
+}
+
+// ----------------------------------------------------------------- batched shared-W projection, complex64
+// part[(p nsys + s)][re | im][Gt] = <W_p, y_s> over a CTA's rows, for p < kk <= 32 and a group of sg
+// systems (blockIdx.y).  Chunks of WD_CH rows of W and of the group's y come in by cp.async, WD_ST deep;
+// lanes are rows, and each of the 24 warps holds one tile of 4 x 4 outputs in registers for all its rows,
+// so a row's 4 + 4 values feed 16 complex products.  With 12 or 6 tiles or fewer, RS = 2 or 4 warps
+// share a tile, each on every RS-th group of 32 rows.  FP32 chains of WD_CHAIN products at most,
+// then the warp's tree, then double-float over the CTAs (k_wdots_reduce).
+constexpr int WD_CH = 128, WD_ST = 3, WD_CHAIN = 128, WD_KMAX = 32, WD_WARPS = 24, WD_NT = WD_WARPS * 32;
+__device__ __forceinline__ void cp_async16z(void *dst, const void *src, int bytes) {   // zero-filled past `bytes`
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(bytes));
+}
+__device__ __forceinline__ void cp_async8z(void *dst, const void *src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(bytes));
+}
+template <int RS>
+__global__ void __launch_bounds__(WD_NT, 1) k_wdots(int n, int kk, const float2 *__restrict__ W,
+                                                    const float2 *__restrict__ Y0, size_t strideY,
+                                                    const int *__restrict__ act, int nsys, int sg, int vec2,
+                                                    double *__restrict__ part) {
+    extern __shared__ __align__(16) float2 wd_sm[];       // [stage][vector][WD_CH]
+    __shared__ int s_act[4 * WD_WARPS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int s0 = blockIdx.y * sg, ns = min(sg, nsys - s0), nv = kk + ns, stage = (kk + sg) * WD_CH;
+    const int tilesP = (kk + 3) / 4, tiles = tilesP * ((ns + 3) / 4);
+    const int tile = warp % tiles, rs = warp / tiles;
+    const bool busy = rs < RS;
+    const int p0 = (tile % tilesP) * 4, c0 = (tile / tilesP) * 4;
+    const int all = (n + WD_CH - 1) / WD_CH;
+    const int nch = (all - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;   // chunks of this CTA
+    if (tid < ns) s_act[tid] = act[s0 + tid];
+    __syncthreads();
+    auto issue = [&](int ch) {
+        if (ch < nch) {
+            float2 *dst = wd_sm + (ch % WD_ST) * stage;
+            const long r0 = ((long)blockIdx.x + (long)ch * gridDim.x) * WD_CH;
+            const int lg = vec2 ? 6 : 7;                  // log2 of the copies a vector takes
+            static_assert(WD_CH == 128, "lg");
+            for (int e = tid; e < nv << lg; e += WD_NT) {
+                const int v = e >> lg, i = (e & ((1 << lg) - 1)) << (7 - lg);
+                const float2 *src = v < kk ? W + (size_t)v * n : Y0 + (size_t)s_act[v - kk] * strideY;
+                const long r = r0 + i;
+                const bool in = r < n;                    // n even with vec2: both elements or neither
+                if (vec2) cp_async16z(dst + v * WD_CH + i, src + (in ? r : 0), in ? 16 : 0);
+                else cp_async8z(dst + v * WD_CH + i, src + (in ? r : 0), in ? 8 : 0);
+            }
+        }
+        cp_async_commit();                                // empty past the end: the group counts stay in step
+    };
+    float2 acc[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[a][c] = make_float2(0.f, 0.f);
+    // the tile's vectors (padding repeats the last one)
+    int wo[4], yo[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        wo[a] = min(p0 + a, kk - 1) * WD_CH + rs * 32 + lane;
+        yo[a] = (kk + min(c0 + a, ns - 1)) * WD_CH + rs * 32 + lane;
+    }
+    for (int ch = 0; ch < WD_ST - 1; ++ch) issue(ch);
+    for (int ch = 0; ch < nch; ++ch) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(WD_ST - 2) : "memory");
+        __syncthreads();                                  // chunk ch landed; the stage refilled below is free
+        issue(ch + WD_ST - 1);
+        if (busy) {
+            const float2 *t = wd_sm + (ch % WD_ST) * stage;
+#pragma unroll
+            for (int i = 0; i < (WD_CH / 32 + RS - 1) / RS; ++i) {
+                if (RS * i + rs < WD_CH / 32) {
+                    float2 w[4], y[4];
+#pragma unroll
+                    for (int a = 0; a < 4; ++a) {
+                        w[a] = t[wo[a] + i * RS * 32];
+                        y[a] = t[yo[a] + i * RS * 32];
+                    }
+#pragma unroll
+                    for (int a = 0; a < 4; ++a)
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) cdotacc(acc[a][c], w[a], y[c]);
+                }
+            }
+        }
+    }
+    if (!busy) return;
+    // reduce-scatter of the 32 sums over the warp: lane l ends with component l = 8 a + 2 c + (re | im)
+    float v[32];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            v[8 * a + 2 * c] = acc[a][c].x;
+            v[8 * a + 2 * c + 1] = acc[a][c].y;
+        }
+#pragma unroll
+    for (int half = 16; half > 0; half >>= 1) {
+        const bool hi = lane & half;
+#pragma unroll
+        for (int q = 0; q < half; ++q) {
+            const float keep = hi ? v[half + q] : v[q], send = hi ? v[q] : v[half + q];
+            v[q] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+        }
+    }
+    const int Gt = gridDim.x * RS, g = blockIdx.x * RS + rs;
+    const int p = p0 + (lane >> 3), c = c0 + ((lane >> 1) & 3);
+    if (p < kk && c < ns)
+        store_df(part + (((size_t)p * nsys + s0 + c) * 2 + (lane & 1)) * Gt + g, dfr(v[0], 0.f));
+}
+// coef_s[p] = the sum over the Gt partials of output (p, s): one warp an output, fixed order.
+__global__ void __launch_bounds__(NT) k_wdots_reduce(int kk, int nsys, int Gt, const double *__restrict__ part,
+                                                     const int *__restrict__ act, double2 *__restrict__ coef0,
+                                                     size_t strideC) {
+    const int lane = threadIdx.x & 31;
+    const int o = blockIdx.x * NW + (threadIdx.x >> 5);
+    if (o >= kk * nsys) return;
+    const double *pp = part + (size_t)o * 2 * Gt;
+    dfr re(0.f, 0.f), im(0.f, 0.f);
+    for (int g = lane; g < Gt; g += 32) {
+        re = re + load_df(pp + g);
+        im = im + load_df(pp + Gt + g);
+    }
+    re = warp_sum(re);
+    im = warp_sum(im);
+    if (lane == 0) coef0[(size_t)act[o % nsys] * strideC + o / nsys] = make_double2((double)re, (double)im);
 }
 
 // ----------------------------------------------------------------- batched update, W in registers
@@ -4481,8 +4591,11 @@ thread_local bool t_capturing = false;   // a stream capture is open on this thr
 // cycle is captured into a CUDA graph.
 int bucket_of(int nsys, int qa, int qb) {
     // a batch against the shared vectors alone (the deflator of the blocked Krylov steps, the deflation
-    // loop's Gram matrix) is its own class, in two for the batches that can and cannot take the tensor cores
-    return (nsys > 1 ? 1 : 0) + (qa > 0 ? 2 : 0) + (nsys > 1 && qa > 0 && qb == 0 ? (nsys >= 8 ? 12 : 4) : 0);
+    // loop's Gram matrix): classes of its own by the batch, since the tensor cores' share of the time
+    // hardly grows with it (at n = 884,736, kk = 24: 173 us for 16 systems, 211 for 64) and the CUDA
+    // cores' does (130 and 367 us)
+    const int wide = nsys < 8 ? 0 : nsys <= 16 ? 1 : nsys <= 32 ? 2 : 3;
+    return (nsys > 1 ? 1 : 0) + (qa > 0 ? 2 : 0) + (nsys > 1 && qa > 0 && qb == 0 ? 4 + 8 * wide : 0);
 }
 
 // A class is tuned on its first launch with at least 8 own-basis vectors (mid-cycle Krylov
@@ -4506,13 +4619,19 @@ int tuned_variant(int prec, int kernel, int n, int nsys, int qa, int qb, int nva
     float best = 1e30f;
     for (int v = 0; v < nvar; ++v) {
         run(v);   // warm
+        // short kernels several times between the events: at ten microseconds the event resolution
+        // alone is more than the 3% that decides below
         float t[3];
-        for (int r = 0; r < 3; ++r) {
+        int reps = 1;
+        for (int r = -1; r < 3; ++r) {
             cudaEventRecord(a, st);
-            run(v);
+            for (int q = 0; q < reps; ++q) run(v);
             cudaEventRecord(b, st);
             cudaEventSynchronize(b);
-            cudaEventElapsedTime(&t[r], a, b);
+            float ms = 0.f;
+            cudaEventElapsedTime(&ms, a, b);
+            if (r < 0) reps = std::max(1, std::min(16, (int)(0.15f / std::max(ms, 1e-3f))));
+            else t[r] = ms / (float)reps;
         }
         std::sort(t, t + 3);
         ent.ms[v] = t[1];
@@ -4653,6 +4772,35 @@ void wproj_run(int n, int kk, const typename CT<R>::t *W, const typename CT<R>::
     k_wproj_reduce<<<(outs + NW - 1) / NW, NT, 0, st>>>(kk, nsys, G, (const double *)partials, act, coef, strideC);
 }
 
+// The complex64 form (k_wdots); false, with nothing launched, where it does not apply or the partial
+// sums do not fit.
+bool wdots_run(int n, int kk, const float2 *W, const float2 *Y, size_t strideY, const int *act, int nsys,
+               double2 *partials, size_t cap, double2 *coef, size_t strideC, cudaStream_t st) {
+    if (kk <= 0 || kk > WD_KMAX || nsys < 2 || n <= 0) return false;
+    // one tile of 4 x 4 outputs a warp; the systems in groups of as many as that allows (32 at most: the
+    // stages' shared memory)
+    const int tilesP = (kk + 3) / 4, sg = std::min(std::min(nsys, 32), 4 * (WD_WARPS / tilesP));
+    const int tiles = tilesP * ((sg + 3) / 4);
+    const int RS = tiles > 12 ? 1 : tiles > 6 ? 2 : 4;
+    const int nch = (n + WD_CH - 1) / WD_CH, groups = (nsys + sg - 1) / sg;
+    // one CTA an SM over the groups, or more where a lane's FP32 chain would pass WD_CHAIN products
+    const int G = std::min(nch, std::max((num_sms() + groups - 1) / groups, (nch * (WD_CH / 32) + WD_CHAIN * RS - 1) / (WD_CHAIN * RS)));
+    if ((size_t)kk * nsys * 2 * RS * G > cap) return false;
+    const int vec2 = n % 2 == 0 && strideY % 2 == 0 && ((uintptr_t)W & 15) == 0 && ((uintptr_t)Y & 15) == 0;
+    const size_t smem = (size_t)WD_ST * (kk + sg) * WD_CH * sizeof(float2);
+    const dim3 grid(G, groups);
+    auto go = [&](auto kernel) {
+        allow_smem(kernel, smem + 1024);   // beside the kernel's static shared memory
+        kernel<<<grid, WD_NT, smem, st>>>(n, kk, W, Y, strideY, act, nsys, sg, vec2, (double *)partials);
+    };
+    if (RS == 4) go(k_wdots<4>);
+    else if (RS == 2) go(k_wdots<2>);
+    else go(k_wdots<1>);
+    k_wdots_reduce<<<(kk * nsys + NW - 1) / NW, NT, 0, st>>>(kk, nsys, G * RS, (const double *)partials, act, coef,
+                                                            strideC);
+    return true;
+}
+
 // W rows held in registers: complex64 up to 32 vectors, complex128 up to 16.
 template <class R> constexpr int wreg_max() { return sizeof(R) == 4 ? 32 : 16; }
 
@@ -4736,8 +4884,14 @@ int mdot_dispatch(int v, int n, const typename CT<R>::t *segA, int qa, const typ
     }
     if (v == VW && !std::is_same<R, dfr>::value) {
         if constexpr (!std::is_same<R, dfr>::value) {
-          if (qa > 0 && batched_w_ok(qa, nsys) && (size_t)qa * nsys * 2 * wproj_grid(n, wp_rt<R>()) <= cap) {
+          bool shared = false;   // the shared part ran on its own
+          if constexpr (sizeof(R) == 4) {
+            shared = qa > 0 && wdots_run(n, qa, segA, w, strideW, act, nsys, partials, cap, coef, strideC, st);
+          } else if (qa > 0 && batched_w_ok(qa, nsys) && (size_t)qa * nsys * 2 * wproj_grid(n, wp_rt<R>()) <= cap) {
             wproj_run<R>(n, qa, segA, w, strideW, act, nsys, partials, coef, strideC, st);
+            shared = true;
+          }
+          if (shared) {
             if (qb == 0) return 2;
             // own-basis part: the tuned choice for a batch without a shared segment
             int vown = 0;
