@@ -119,7 +119,7 @@ __device__ __forceinline__ float scatter12(float (&v)[12], int lane) {
     return c[0] + __shfl_xor_sync(0xffffffffu, c[0], 1);
 }
 
-// part[slot][6 i + 2 b + (re | im)][G]: <v_i, y_b> for the nv basis vectors, then <y_a, y_b>; y_b is
+// part[slot][G][6 i + 2 b + (re | im)]: <v_i, y_b> for the nv basis vectors, then <y_a, y_b>; y_b is
 // basis slot nv + b.  HBM-bound: a CTA keeps the block's elements of a chunk in registers and streams
 // the basis past them two vectors at a time.  FP32 sums over 256 elements a warp, then double-float.
 template <int EPT, int VEC>
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(NTB, 2)
         dfr t(0.f, 0.f);
 #pragma unroll
         for (int w = 0; w < NWB; ++w) t = t + bp_ws[(size_t)w * ncomp + c];
-        *reinterpret_cast<dfr *>(pp + (size_t)c * G + blockIdx.y) = t;
+        *reinterpret_cast<dfr *>(pp + (size_t)blockIdx.y * ncomp + c) = t;
     }
 }
 
@@ -277,7 +277,8 @@ __device__ __forceinline__ double wsum(double v) {
 
 // One CTA a system: the block's coefficients from the partial sums, the Cholesky factor, the
 // update's coefficients (dco: T then D) and the block's Hessenberg columns.  Latency-bound.
-__global__ void __launch_bounds__(NTB) k_block_finish(int nv, int kk, int m, int G, const double *__restrict__ part,
+constexpr int NTF = 512;
+__global__ void __launch_bounds__(NTF) k_block_finish(int nv, int kk, int m, int G, const double *__restrict__ part,
                                                       const int *__restrict__ act, SysState *state,
                                                       double2 *__restrict__ H0, size_t strideH,
                                                       const double2 *__restrict__ a0, const double2 *__restrict__ a1,
@@ -294,27 +295,41 @@ __global__ void __launch_bounds__(NTB) k_block_finish(int nv, int kk, int m, int
     const int ncomp = BK_C * (nv + BK_S), nown = nv + BK_S;
     if (stt.broken) {
         if (tid < BK_S * BK_S) d[tid] = make_float2(0.f, 0.f);
-        for (int i = tid; i < BK_S * nv; i += NTB) d[BK_S * BK_S + i] = make_float2(0.f, 0.f);
+        for (int i = tid; i < BK_S * nv; i += NTF) d[BK_S * BK_S + i] = make_float2(0.f, 0.f);
         return;
     }
+    // the CTAs' sums: a thread a component (coalesced across components), the CTAs split over as many
+    // thread groups as fit, four loads in flight, then the groups in order.  (A warp a component, a
+    // butterfly each, was most of 38 us a block for 16 systems at 64^3.)
     const double *pp = part + (size_t)slot * ncomp * G;
-    for (int c = warp; c < ncomp; c += NWB) {
+    __shared__ dfr gsum[NTF];
+    const int per = ncomp < NTF ? ncomp : NTF, groups = NTF / per, grp = tid / per;
+    for (int c0 = 0; c0 < ncomp; c0 += per) {
+        const int c = c0 + tid % per;
         dfr t(0.f, 0.f);
-        for (int g = lane; g < G; g += 32) {
-            const float2 f = __ldcg(reinterpret_cast<const float2 *>(pp + (size_t)c * G + g));
-            t = t + dfr(f.x, f.y);
-        }
+        if (grp < groups && c < ncomp)
+            for (int g = grp; g < G; g += 4 * groups) {
+                float2 f[4];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            t = t + dfr(__shfl_xor_sync(0xffffffffu, t.hi, o), __shfl_xor_sync(0xffffffffu, t.lo, o));
-        if (lane == 0) {
+                for (int u = 0; u < 4; ++u)
+                    f[u] = g + u * groups < G
+                               ? __ldcg(reinterpret_cast<const float2 *>(pp + (size_t)(g + u * groups) * ncomp + c))
+                               : make_float2(0.f, 0.f);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) t = t + dfr(f[u].x, f[u].y);
+            }
+        gsum[tid] = t;
+        __syncthreads();
+        if (grp == 0 && c < ncomp) {
+            for (int h = 1; h < groups; ++h) t = t + gsum[h * per + tid];
             const int i = c / BK_C, b = (c % BK_C) >> 1;
             double2 &z = i < nv ? q[b + 1][i] : gs[i - nv][b];
             if (c & 1) z.y = (double)t;
             else z.x = (double)t;
         }
+        __syncthreads();
     }
-    for (int i = tid; i < nown; i += NTB) q[0][i] = make_double2(i == nv - 1 ? 1.0 : 0.0, 0.0);
+    for (int i = tid; i < nown; i += NTF) q[0][i] = make_double2(i == nv - 1 ? 1.0 : 0.0, 0.0);
     __syncthreads();
     // G - C^H C, upper triangle, one warp an entry
     if (warp < 6) {
@@ -330,7 +345,7 @@ __global__ void __launch_bounds__(NTB) k_block_finish(int nv, int kk, int m, int
         if (lane == 0) ss[a][b] = make_double2(gs[a][b].x - z.x, gs[a][b].y - z.y);
     }
     __syncthreads();
-    const double sig = (double)stt.bs_sigma;
+    const double sig = (double)stt.bs_sigma, isig = 1.0 / sig;
     const double2 th = make_double2((double)stt.bs_tr, (double)stt.bs_ti);
     if (tid == 0) {
         bool ok = true;
@@ -349,11 +364,10 @@ __global__ void __launch_bounds__(NTB) k_block_finish(int nv, int kk, int m, int
             for (int l = 0; l < b; ++l) piv -= r[l][b].x * r[l][b].x + r[l][b].y * r[l][b].y;
             // also false for NaN and for an infinite column norm
             if (!(piv > BK_ILL * gs[b][b].x) || !(gs[b][b].x < 1e30)) ok = false;
-            const double rr = ok ? sqrt(piv) : 1.0;
-            ri[b] = 1.0 / rr;
-            r[b][b] = make_double2(rr, 0.0);
+            ri[b] = ok ? rsqrt(piv) : 1.0;
+            r[b][b] = make_double2(ok ? piv * ri[b] : 1.0, 0.0);
             // the subdiagonal of the column this vector completes, in the operator's units
-            const double beta = b == 0 ? rr / sig : rr * ri[b - 1] / sig;
+            const double beta = r[b][b].x * isig * (b == 0 ? 1.0 : ri[b - 1]);
             if (!(beta >= tol) || !(beta < 1e300)) ok = false;
         }
         // T = R^-1, upper triangular
@@ -378,27 +392,26 @@ __global__ void __launch_bounds__(NTB) k_block_finish(int nv, int kk, int m, int
     __syncthreads();
     if (!s_ok) {
         if (tid < BK_S * BK_S) d[tid] = make_float2(0.f, 0.f);
-        for (int i = tid; i < BK_S * nv; i += NTB) d[BK_S * BK_S + i] = make_float2(0.f, 0.f);
+        for (int i = tid; i < BK_S * nv; i += NTF) d[BK_S * BK_S + i] = make_float2(0.f, 0.f);
         return;
     }
     if (tid < BK_S * BK_S) {
         const double2 t = tt[tid / BK_S][tid % BK_S];
         d[tid] = make_float2((float)t.x, (float)t.y);
     }
-    for (int e = tid; e < BK_S * nv; e += NTB) {   // D = C T
+    for (int e = tid; e < BK_S * nv; e += NTF) {   // D = C T
         const int i = e / BK_S, b = e % BK_S;
         double2 z = make_double2(0.0, 0.0);
         for (int a = 0; a <= b; ++a) z = zfma(q[a + 1][i], tt[a][b], z);
         d[BK_S * BK_S + e] = make_float2((float)z.x, (float)z.y);
     }
-    // the columns nv - 1 + b of A V = [W V] H: four lanes a row, row = tid / 4, tid / 4 + 64, ...
-    const double isig = 1.0 / sig;
+    // the columns nv - 1 + b of A V = [W V] H: four lanes a row, row = tid / 4, tid / 4 + NTF / 4, ...
     const int part4 = tid & 3;
     for (int b = 0; b < BK_S; ++b) {
         const int col = nv - 1 + b;                       // own column; rows kk + 0 .. col + 1
         const double2 *ab = (b == 0 ? a0 : b == 1 ? a1 : a2) + (size_t)s * strideC;
         const double ir = tt[b > 0 ? b - 1 : 0][b > 0 ? b - 1 : 0].x;   // 1 / R_bb of q[b] (b > 0)
-        for (int r0 = tid >> 2; r0 < ((kk + col + 2 + 63) & ~63); r0 += 64) {   // warp-uniform trip count
+        for (int r0 = tid >> 2; r0 < ((kk + col + 2 + NTF / 4 - 1) & ~(NTF / 4 - 1)); r0 += NTF / 4) {   // warp-uniform
             double2 z = make_double2(0.0, 0.0);
             const int own = r0 - kk;
             if (b > 0 && r0 < kk + col + 2)
@@ -426,7 +439,7 @@ __global__ void __launch_bounds__(NTB) k_block_finish(int nv, int kk, int m, int
                 H[(size_t)(kk + col) * ld + r0] = z;
             }
         }
-        for (int r0 = kk + col + 2 + tid; r0 < kk + nown + 1; r0 += NTB) hc[b][r0] = make_double2(0.0, 0.0);
+        for (int r0 = kk + col + 2 + tid; r0 < kk + nown + 1; r0 += NTF) hc[b][r0] = make_double2(0.0, 0.0);
         __syncthreads();
     }
     if (tid == 0) {
@@ -514,7 +527,7 @@ void launch_block_step(int n, int nv, int kk, int m, float2 *V, size_t strideV, 
         };
         if (ept == EPT_BIG) v2 ? go(k_block_proj<EPT_BIG, 2>) : go(k_block_proj<EPT_BIG, 1>);
         else v2 ? go(k_block_proj<EPT_SMALL, 2>) : go(k_block_proj<EPT_SMALL, 1>);
-        k_block_finish<<<nsys, NTB, 0, st>>>(nv, kk, m, G, scratch, act, state, H, strideH, a[0], a[1], a[2], strideC, tol,
+        k_block_finish<<<nsys, NTF, 0, st>>>(nv, kk, m, G, scratch, act, state, H, strideH, a[0], a[1], a[2], strideC, tol,
                                              dco, dstride);
     }
     ProfScope p(KC_UPDATE, sizeof(float2) * (double)n * nsys * (nv + 2 * BK_S), st, 1);
