@@ -642,7 +642,7 @@ template <class R> int Engine<R>::run_cycle(int kk, int nsys, int lead, double t
     cudaGraphExec_t exec = nullptr;
     for (auto &g : graphs_)
         if (g.kk == kk && g.nsys == nsys && g.zpar == zpar && g.tol == tol && g.blocked == blocked_ &&
-            g.cholqr == cholqr_on_)
+            g.cholqr == cholqr_on_ && g.gdirect == g_direct_)
             exec = g.exec;
     if (!exec) {
         if (graphs_.size() >= 32) {
@@ -670,7 +670,7 @@ template <class R> int Engine<R>::run_cycle(int kk, int nsys, int lead, double t
             set_last_error(GDMR_ECUDA, std::string("restart-cycle graph: ") + cudaGetErrorString(e));
             return GDMR_ECUDA;
         }
-        graphs_.push_back(GraphEntry{kk, nsys, zpar, tol, blocked_, cholqr_on_, exec});
+        graphs_.push_back(GraphEntry{kk, nsys, zpar, tol, blocked_, cholqr_on_, g_direct_, exec});
     }
     GDMR_CK(cudaGraphLaunch(exec, stream));
     // the graph joins the deflation update into the main stream: the new Z is ready in order
@@ -722,6 +722,7 @@ template <class R> int Engine<R>::enqueue_front(int kk, int nsys, long *matvecs)
     } else if (hook) {
         cudaMemcpyAsync(op.ext, V_, sizeof(C) * n, cudaMemcpyDeviceToDevice, stream);
     }
+    if (g_direct_) launch_unit_coordinates(m, kk, coef_, g_, sC, act_, nsys, state_, stream);
     GDMR_CK(cudaGetLastError());
     return GDMR_OK;
 }
@@ -890,8 +891,8 @@ template <class R> int Engine<R>::enqueue_krylov_blocked(int kk, int nsys, doubl
             launch_scale<R>(n, T_, n, slot, sV, nullptr, 0, act_, nsys, state_, true, stream);
         }
         launch_block_init(first, kk, m, act_, nsys, state_, H_, strideH(), stream);
-        double2 *a[KRYLOV_BLOCK] = {g_, y_, t_};   // free until the cycle's end
-        const double2 *ac[KRYLOV_BLOCK] = {g_, y_, t_};
+        double2 *a[KRYLOV_BLOCK] = {coef_, y_, t_};   // y_ and t_ are free until the cycle's end
+        const double2 *ac[KRYLOV_BLOCK] = {coef_, y_, t_};
         for (int nv = first + 1; nv + KRYLOV_BLOCK <= steps + 1; nv += KRYLOV_BLOCK) {
             for (int b = 0; b < KRYLOV_BLOCK; ++b)
                 product(V_ + (size_t)(nv - 1 + b) * n, V_ + (size_t)(nv + b) * n, true, a[b]);
@@ -922,8 +923,9 @@ template <class R> int Engine<R>::enqueue_back(int kk, int nsys, bool join) {
         z_pending_ = true;
     }
     // g = [W V]^H r (updateTrgCoeffsDMR, gDMR.cu:2334-2408)
-    launch_mdot<R>(n, W_, kk, V_, sV, m + 1 - kk, R_, n, act_, nsys, partials_, qmax(), tickets_, g_, sC, state_, false,
-                   stream);
+    if (!g_direct_)
+        launch_mdot<R>(n, W_, kk, V_, sV, m + 1 - kk, R_, n, act_, nsys, partials_, qmax(), tickets_, g_, sC, state_,
+                       false, stream);
     // y = argmin ||H y - g||, t = H y (qrHessArrDMR/qrSolveDMR/hessenbergMultDMR)
     launch_ls(m, H_, strideH(), g_, y_, t_, sC, act_, nsys, stream);
     // r -= [W V] t ; x += rho_abs [Z V] y ; rho = ||r|| (updateAppResDMR, gDMR.cu:2411-2582)
@@ -1113,16 +1115,21 @@ int Engine<R>::refine_admit(int slot, const double2 *b, const double2 *x0, doubl
 // The stagnation rule of the restart (arnoldiSetupDMR, gDMR.cu:2600-2621): a system whose last
 // cycle stagnated starts from the Krylov vector at storage index kk + (m - k)/2 of that cycle
 // instead of from the unit residual, which k_demote_unit has already written as basis vector 0.
-template <class R> void Engine<R>::restart_vectors(const std::vector<int> &next, int kk) {
+// Returns whether any system did.
+template <class R> bool Engine<R>::restart_vectors(const std::vector<int> &next, int kk) {
     const int n = n_, m = m_, k = k_;
+    bool any = false;
     for (int s : next) {
         Slot &S = slot_[s];
         const int period = (2 * S.max_cycles) / (m - k);
         if (S.loop_flag == 0 || (period != 0 && S.flag_count % period == 0)) continue;
         const int idx = kk + (m - k) / 2 - kk_prev_;
-        if (idx > 0 && idx <= m)
+        if (idx > 0 && idx <= m) {
             cudaMemcpyAsync(Vs(s), Vs(s) + (size_t)idx * n, sizeof(C) * n, cudaMemcpyDeviceToDevice, stream);
+            any = true;
+        }
     }
+    return any;
 }
 
 template <class R> int Engine<R>::refine_cycle(std::vector<int> *done) {
@@ -1217,14 +1224,14 @@ template <class R> int Engine<R>::refine_cycle(std::vector<int> *done) {
     k_cycle_reset<<<1, 256, 0, stream>>>(act_, na, state_, 1);
     const int kk = (k > 0 && have_z_) ? k : 0;
     if (kk == 0) front_done_ = false;   // the deflation space was dropped after a timeout
-    restart_vectors(next, kk);
+    g_direct_ = !restart_vectors(next, kk);
     long mv = 0;
     // breakdown of unit vectors: an invariant subspace at working precision
     const double inner_tol = sizeof(R) == 4 ? 1e-6 : 1e-14;
     blocked_ = blocks_on_;
     const bool had_z = have_z_;
     const int cycle_rc = run_cycle(kk, na, lead, inner_tol, &mv);
-    blocked_ = false;
+    blocked_ = g_direct_ = false;
     if (cycle_rc != GDMR_OK) return GDMR_ECUDA;
     launch_refine_update<R>(n, x64_, n, X_, n, act_, na, state_, cap_, stream);
     if (read_state(cap_ + 1) != GDMR_OK) return GDMR_ECUDA;

@@ -171,7 +171,7 @@ template <class R> class Engine {
     // multi_jobs appends one Krylov job per such system; multi_back waits for the event `after`
     // (the launch) and enqueues the rest of the cycle and the FP64 correction.  SELL operators.
     int multi_residual();
-    void restart_vectors(const std::vector<int> &next, int kk);
+    bool restart_vectors(const std::vector<int> &next, int kk);
     int multi_select(std::vector<int> *done);
     int multi_front();
     void multi_jobs(std::vector<KrylovJob<R>> &jobs) const;
@@ -260,7 +260,7 @@ template <class R> class Engine {
     struct GraphEntry {
         int kk, nsys, zpar;
         double tol;
-        bool blocked, cholqr;
+        bool blocked, cholqr, gdirect;
         cudaGraphExec_t exec;
     };
     std::vector<GraphEntry> graphs_;
@@ -276,6 +276,9 @@ template <class R> class Engine {
     // Cholesky QR in the deflation loop: refined_ is set around refined cycles, cholqr_on_ until a factor
     // breaks down.
     bool refined_ = false, cholqr_on_ = true;
+    // The cycle's systems all start from their residuals, so the residuals' coordinates in [W V] are known
+    // without a pass over the basis (launch_unit_coordinates).
+    bool g_direct_ = false;
     bool cholqr_ok(int kk) const;
     void enqueue_deflation_cholqr(int kk, long *matvecs);
     bool blocked_ok(int kk, int nsys) const;

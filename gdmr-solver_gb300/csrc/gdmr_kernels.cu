@@ -2865,84 +2865,89 @@ __global__ void __launch_bounds__(NT) k_znormalise(int n, const typename CT<R>::
 // memory at off(c) = c(c+3)/2, rows 0..c+1.
 __device__ __forceinline__ int hoff(int c) { return c * (c + 3) / 2; }
 
-__global__ void __launch_bounds__(128) k_ls(int m, const double2 *__restrict__ H0, size_t strideH,
+// One CTA a system, thread c on column c (thread m on g).  Latency-bound: m dependent rotations, then m
+// dependent back-substitution steps, all FP64, whose instructions take about 20 SM clocks a warp on
+// GB300.  So the rotation is the complex one [conj a, conj b; -b, a] / r, r = (|a|^2 + |b|^2)^(1/2): one
+// reciprocal square root a step (three hypots and five divisions before), R's diagonal is real, and each
+// phase synchronises once a step: m = 48, 16 systems: 266 to 108 us.
+__global__ void __launch_bounds__(192) k_ls(int m, const double2 *__restrict__ H0, size_t strideH,
                                             const double2 *__restrict__ g0, double2 *__restrict__ y0,
                                             double2 *__restrict__ t0, size_t strideC, const int *__restrict__ act) {
     extern __shared__ double2 sm[];
     const int s = act[blockIdx.x], tid = threadIdx.x, ld = m + 1;
     const double2 *H = H0 + (size_t)s * strideH;
     double2 *Hp = sm;                         // packed Hessenberg
-    double2 *gg = sm + hoff(m);               // m+1
+    double2 *gg = sm + hoff(m);               // m+1: column m of the same packing
     double2 *yy = gg + (m + 1);               // m
-    double *cs = (double *)(yy + m);          // m cosines
-    double2 *sn = (double2 *)(cs + m + (m & 1));   // m sines (keep 16-byte alignment)
-    for (int c = 0; c < m; ++c)
-        for (int r = tid; r <= c + 1 && r <= m; r += blockDim.x) Hp[hoff(c) + r] = H[(size_t)c * ld + r];
+    double2 *ra = yy + m, *rb = ra + m;       // rotations
+    double *iv = (double *)(rb + m);          // 1 / R[i][i] (0 for a zero pivot)
+    for (int e = tid; e < m * ld; e += blockDim.x) {
+        const int c = e / ld, r = e - c * ld;
+        if (r <= c + 1) Hp[hoff(c) + r] = H[e];
+    }
     for (int r = tid; r <= m; r += blockDim.x) gg[r] = g0[(size_t)s * strideC + r];
     __syncthreads();
+    double2 *col = Hp + hoff(tid);            // gg for thread m
     for (int i = 0; i < m; ++i) {
-        if (tid == 0) {
-            double2 a = Hp[hoff(i) + i], b = Hp[hoff(i) + i + 1];
-            double aa = hypot(a.x, a.y), bb = hypot(b.x, b.y);
-            double c, rr;
-            double2 sv, ph;
-            if (bb == 0.0) {
-                c = 1.0; sv = make_double2(0, 0); rr = aa; ph = aa > 0 ? make_double2(a.x / aa, a.y / aa) : make_double2(1, 0);
-            } else if (aa == 0.0) {
-                c = 0.0; sv = make_double2(b.x / bb, -b.y / bb); rr = bb; ph = make_double2(1, 0);
-            } else {
-                double rho = hypot(aa, bb);
-                ph = make_double2(a.x / aa, a.y / aa);
-                c = aa / rho;
-                // s = ph * conj(b) / rho
-                sv = make_double2((ph.x * b.x + ph.y * b.y) / rho, (ph.y * b.x - ph.x * b.y) / rho);
-                rr = rho;
+        if (tid == i) {
+            double2 a = col[i], b = col[i + 1];
+            double n2 = a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y, scale = 1.0;
+            if (!(n2 > 1e-280 && n2 < 1e280)) {   // squares out of range (or not a number): scaled first
+                const double mx = fmax(fmax(fabs(a.x), fabs(a.y)), fmax(fabs(b.x), fabs(b.y)));
+                if (mx > 0.0 && mx < 1.7e308) {
+                    scale = 1.0 / mx;
+                    if (!(scale < 1e308)) scale = 1e308;   // mx denormal
+                    a = make_double2(a.x * scale, a.y * scale);
+                    b = make_double2(b.x * scale, b.y * scale);
+                    n2 = a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y;
+                }
             }
-            cs[i] = c;
-            sn[i] = sv;
-            Hp[hoff(i) + i] = make_double2(ph.x * rr, ph.y * rr);
-            Hp[hoff(i) + i + 1] = make_double2(0, 0);
-            double2 g1 = gg[i], g2 = gg[i + 1];
-            // [c s; -conj(s) c] [g1; g2]
-            gg[i] = make_double2(c * g1.x + sv.x * g2.x - sv.y * g2.y, c * g1.y + sv.x * g2.y + sv.y * g2.x);
-            gg[i + 1] = make_double2(-(sv.x * g1.x + sv.y * g1.y) + c * g2.x, -(sv.x * g1.y - sv.y * g1.x) + c * g2.y);
+            if (n2 == 0.0) {
+                ra[i] = make_double2(1.0, 0.0);
+                rb[i] = make_double2(0.0, 0.0);
+                iv[i] = 0.0;
+            } else {
+                const double inv = rsqrt(n2);
+                ra[i] = make_double2(a.x * inv, a.y * inv);
+                rb[i] = make_double2(b.x * inv, b.y * inv);
+                iv[i] = inv * scale;
+            }
         }
         __syncthreads();
-        const double c = cs[i];
-        const double2 sv = sn[i];
-        for (int col = i + 1 + tid; col < m; col += blockDim.x) {
-            double2 h1 = Hp[hoff(col) + i], h2 = Hp[hoff(col) + i + 1];
-            Hp[hoff(col) + i] = make_double2(c * h1.x + sv.x * h2.x - sv.y * h2.y, c * h1.y + sv.x * h2.y + sv.y * h2.x);
-            Hp[hoff(col) + i + 1] = make_double2(-(sv.x * h1.x + sv.y * h1.y) + c * h2.x, -(sv.x * h1.y - sv.y * h1.x) + c * h2.y);
+        if (tid > i && tid <= m) {
+            const double2 a = ra[i], b = rb[i], h1 = col[i], h2 = col[i + 1];
+            col[i] = make_double2(a.x * h1.x + a.y * h1.y + b.x * h2.x + b.y * h2.y,
+                                  a.x * h1.y - a.y * h1.x + b.x * h2.y - b.y * h2.x);
+            col[i + 1] = make_double2(a.x * h2.x - a.y * h2.y - b.x * h1.x + b.y * h1.y,
+                                      a.x * h2.y + a.y * h2.x - b.x * h1.y - b.y * h1.x);
         }
-        __syncthreads();
     }
-    // back substitution R y = g (R = upper m x m part); zero pivots give zero components
+    __syncthreads();
+    // back substitution R y = g, thread r on row r; zero pivots give zero components
+    double2 g = tid < m ? gg[tid] : make_double2(0.0, 0.0);
+    const double rd = tid < m && iv[tid] != 0.0 ? 1.0 / iv[tid] : 0.0;   // R[tid][tid]
     for (int c = m - 1; c >= 0; --c) {
-        if (tid == 0) {
-            double2 d = Hp[hoff(c) + c], g = gg[c];
-            double dd = d.x * d.x + d.y * d.y;
-            yy[c] = dd > 0 ? make_double2((g.x * d.x + g.y * d.y) / dd, (g.y * d.x - g.x * d.y) / dd) : make_double2(0, 0);
-        }
+        if (tid == c) yy[c] = rd == 0.0 ? make_double2(0.0, 0.0) : make_double2(g.x / rd, g.y / rd);
         __syncthreads();
-        const double2 yc = yy[c];
-        for (int r = tid; r < c; r += blockDim.x) {
-            double2 h = Hp[hoff(c) + r];
-            gg[r].x -= h.x * yc.x - h.y * yc.y;
-            gg[r].y -= h.x * yc.y + h.y * yc.x;
+        if (tid < c) {
+            const double2 h = Hp[hoff(c) + tid], yc = yy[c];
+            g.x -= h.x * yc.x - h.y * yc.y;
+            g.y -= h.x * yc.y + h.y * yc.x;
         }
-        __syncthreads();
     }
     for (int c = tid; c < m; c += blockDim.x) y0[(size_t)s * strideC + c] = yy[c];
-    // t = H y with the original H
+    // t = H y with the original H, two chains a row
     for (int r = tid; r <= m; r += blockDim.x) {
-        double2 acc = make_double2(0, 0);
-        for (int c = (r > 0 ? r - 1 : 0); c < m; ++c) {
-            double2 h = H[(size_t)c * ld + r], yc = yy[c];
-            acc.x += h.x * yc.x - h.y * yc.y;
-            acc.y += h.x * yc.y + h.y * yc.x;
+        double2 acc[2] = {make_double2(0, 0), make_double2(0, 0)};
+        int u = 0;
+#pragma unroll 4
+        for (int c = (r > 0 ? r - 1 : 0); c < m; ++c, u ^= 1) {
+            const double2 h = H[(size_t)c * ld + r], yc = yy[c];
+            double2 &z = acc[u];
+            z.x += h.x * yc.x - h.y * yc.y;
+            z.y += h.x * yc.y + h.y * yc.x;
         }
-        t0[(size_t)s * strideC + r] = acc;
+        t0[(size_t)s * strideC + r] = make_double2(acc[0].x + acc[1].x, acc[0].y + acc[1].y);
     }
 }
 
@@ -2973,90 +2978,111 @@ __device__ __forceinline__ void circle_pair(int r, int pi, int mm, int &p, int &
 }
 
 // QR with column pivoting (Businger and Golub 1965) of A ((m+1) x m, column-major, FP32) in
-// place, by Householder reflections in the conventions of LAPACK's xLARFG: on return the upper
-// triangle holds R, and column j of R comes from column perm[j] of A.  Pivoting on the largest
+// place, by Householder reflections in the conventions of LAPACK's xLARFG: on return column perm[j] of
+// the array holds, in its rows 0..j, column j of R.  Pivoting on the largest
 // remaining column norm grades R, which lets one-sided Jacobi on R^H converge in about half
 // the sweeps it takes on A (Drmac and Veselic 2008).  The partial norms are recomputed after
-// each step, not downdated.  pn (m) is scratch; s_c a shared scalar.
-__device__ void qrcp_f32(int m, float2 *A, int *perm, float *pn, float2 *s_c) {
+// each step, not downdated.  Columns stay where they are (a norm below zero marks a finished one), and
+// every warp finds the pivot and forms its reflector for itself, in registers: one barrier a step, with
+// the norms double-buffered.  (One warp at both, with the columns swapped, took 4100 of k_svd's clocks a
+// step at m = 48.)  pna, pnb: m floats of scratch each; RPL: rows a lane, 32 RPL >= m + 1.
+template <int RPL> __device__ void qrcp_f32(int m, float2 *A, int *perm, float *pna, float *pnb) {
     const int rows = m + 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
     for (int c = warp; c < m; c += nwarps) {
         float a = 0.f;
         for (int r = lane; r < rows; r += 32) { const float2 v = A[(size_t)c * rows + r]; a += v.x * v.x + v.y * v.y; }
         a = warp_sum(a);
-        if (lane == 0) { pn[c] = a; perm[c] = c; }
+        if (lane == 0) pna[c] = a;
     }
     __syncthreads();
+    int done = -1;             // the last step's pivot column, whose diagonal is still to be stored
+    float2 diag = make_float2(0.f, 0.f);
     for (int j = 0; j < m; ++j) {
-        float2 *aj = A + (size_t)j * rows;
-        if (warp == 0) {
-            // pivot: the largest remaining norm, lowest index on ties; swap it into column j
-            float best = -1.f;
-            int bi = j;
-            for (int c = j + lane; c < m; c += 32)
-                if (pn[c] > best) { best = pn[c]; bi = c; }
-            for (int o = 16; o > 0; o >>= 1) {
-                const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-            }
-            if (bi != j) {
-                float2 *ap = A + (size_t)bi * rows;
-                for (int r = lane; r < rows; r += 32) { const float2 t = aj[r]; aj[r] = ap[r]; ap[r] = t; }
-                if (lane == 0) {
-                    const int t = perm[j]; perm[j] = perm[bi]; perm[bi] = t;
-                    const float u = pn[j]; pn[j] = pn[bi]; pn[bi] = u;
-                }
-                __syncwarp();
-            }
-            // reflector H = I - tau v v^H, v = (1, x / (alpha - beta))
-            float xn = 0.f;
-            for (int r = j + 1 + lane; r < rows; r += 32) xn += aj[r].x * aj[r].x + aj[r].y * aj[r].y;
-            xn = warp_sum(xn);
-            const float2 al = aj[j];
-            float2 tau = make_float2(0.f, 0.f);
-            if (xn > 0.f || al.y != 0.f) {
-                const float beta = -copysignf(sqrtf(al.x * al.x + al.y * al.y + xn), al.x);
-                tau = make_float2((beta - al.x) / beta, -al.y / beta);
-                const float2 d = make_float2(al.x - beta, al.y);                  // 1 / (alpha - beta)
-                const float id = 1.f / (d.x * d.x + d.y * d.y);
-                const float2 sc = make_float2(d.x * id, -d.y * id);
-                for (int r = j + 1 + lane; r < rows; r += 32) {
-                    const float2 x = aj[r];
-                    aj[r] = make_float2(x.x * sc.x - x.y * sc.y, x.x * sc.y + x.y * sc.x);
-                }
-                __syncwarp();
-                if (lane == 0) aj[j] = make_float2(beta, 0.f);
-            }
-            if (lane == 0) *s_c = tau;
+        const float *pn = j & 1 ? pnb : pna;
+        float *pw = j & 1 ? pna : pnb;
+        if (done >= 0 && tid == 0) A[(size_t)done * rows + j - 1] = diag;   // every warp has read the column
+        // pivot: the largest remaining norm, lowest index on ties
+        float best = -1.f;
+        int bi = m;
+        for (int c = lane; c < m; c += 32)
+            if (pn[c] > best) { best = pn[c]; bi = c; }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+            if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
         }
-        __syncthreads();
-        const float2 tau = *s_c;
-        for (int c = j + 1 + warp; c < m; c += nwarps) {   // a_c <- (I - conj(tau) v v^H) a_c
+        if (bi >= m) {   // no norm compares (NaN): the first column not finished, the same in every warp
+            for (int c = m - 1; c >= 0; --c)
+                if (!(pn[c] < 0.f)) bi = c;
+        }
+        if (warp == 0 && lane == 0) perm[j] = bi;
+        // reflector H = I - tau v v^H, v = (1, x / (alpha - beta)), from the pivot column's rows j..m
+        float2 *aj = A + (size_t)bi * rows;
+        float2 v[RPL];
+        float xn = 0.f;
+#pragma unroll
+        for (int u = 0; u < RPL; ++u) {
+            const int r = lane + 32 * u;
+            v[u] = (r >= j && r < rows) ? aj[r] : make_float2(0.f, 0.f);
+            if (r > j) xn += v[u].x * v[u].x + v[u].y * v[u].y;
+        }
+        xn = warp_sum(xn);
+        const float2 al = aj[j];
+        float2 tau = make_float2(0.f, 0.f), sc = make_float2(0.f, 0.f);
+        float beta = al.x;
+        const bool refl = xn > 0.f || al.y != 0.f;
+        if (refl) {
+            beta = -copysignf(sqrtf(al.x * al.x + al.y * al.y + xn), al.x);
+            const float ib = 1.f / beta;
+            tau = make_float2((beta - al.x) * ib, -al.y * ib);
+            const float2 d = make_float2(al.x - beta, al.y);                  // 1 / (alpha - beta)
+            const float id = 1.f / (d.x * d.x + d.y * d.y);
+            sc = make_float2(d.x * id, -d.y * id);
+        }
+#pragma unroll
+        for (int u = 0; u < RPL; ++u) {
+            const int r = lane + 32 * u;
+            const float2 x = v[u];
+            v[u] = r == j ? make_float2(1.f, 0.f)
+                          : r > j ? make_float2(x.x * sc.x - x.y * sc.y, x.x * sc.y + x.y * sc.x) : make_float2(0.f, 0.f);
+        }
+        for (int c = warp; c < m; c += nwarps) {   // a_c <- (I - conj(tau) v v^H) a_c
+            if (c == bi || pn[c] < 0.f) {
+                if (lane == 0) pw[c] = -1.f;
+                continue;
+            }
             float2 *ac = A + (size_t)c * rows;
+            float2 a[RPL];
             float wr = 0.f, wi = 0.f;
-            for (int r = j + lane; r < rows; r += 32) {
-                const float2 v = (r == j) ? make_float2(1.f, 0.f) : aj[r], a = ac[r];
-                wr += v.x * a.x + v.y * a.y;
-                wi += v.x * a.y - v.y * a.x;
+#pragma unroll
+            for (int u = 0; u < RPL; ++u) {
+                const int r = lane + 32 * u;
+                a[u] = (r >= j && r < rows) ? ac[r] : make_float2(0.f, 0.f);
+                wr += v[u].x * a[u].x + v[u].y * a[u].y;
+                wi += v[u].x * a[u].y - v[u].y * a[u].x;
             }
             wr = warp_sum(wr);
             wi = warp_sum(wi);
             const float fr = tau.x * wr + tau.y * wi, fi = tau.x * wi - tau.y * wr;   // conj(tau) w
             float s = 0.f;
-            for (int r = j + lane; r < rows; r += 32) {
-                const float2 v = (r == j) ? make_float2(1.f, 0.f) : aj[r];
-                float2 a = ac[r];
-                a.x -= fr * v.x - fi * v.y;
-                a.y -= fr * v.y + fi * v.x;
-                ac[r] = a;
-                if (r > j) s += a.x * a.x + a.y * a.y;
+#pragma unroll
+            for (int u = 0; u < RPL; ++u) {
+                const int r = lane + 32 * u;
+                a[u].x -= fr * v[u].x - fi * v[u].y;
+                a[u].y -= fr * v[u].y + fi * v[u].x;
+                if (r >= j && r < rows) ac[r] = a[u];
+                if (r > j) s += a[u].x * a[u].x + a[u].y * a[u].y;
             }
             s = warp_sum(s);
-            if (lane == 0) pn[c] = s;
+            if (lane == 0) pw[c] = s;
         }
+        done = bi;
+        diag = make_float2(refl ? beta : al.x, refl ? 0.f : al.y);
         __syncthreads();
     }
+    if (tid == 0) A[(size_t)done * rows + m - 1] = diag;
+    __syncthreads();
 }
 
 // The circle schedule as a table: entry round * (mm/2) + pi = p | q << 8 (p < q < mm <= 256).
@@ -3170,6 +3196,122 @@ __device__ int jacobi_sweeps_f32(int m, int rows, float2 *A, float2 *V, float *n
     return sweep + 1;
 }
 
+// jacobi_sweeps_f32 without V for rows = m <= 64 and a warp a pair: each warp keeps its two columns in
+// registers, two rows a lane, and a round hands them on through shared memory along the circle (the top
+// row to the right, the bottom row to the left), double-buffered in `ex` (2 x mm columns of m float2, mm = m
+// rounded up to even).  One barrier a round, the columns read and written once (the in-place form reads them twice:
+// 2100 clocks a round at m = 48, bound by its instructions).  A column's squared norm and id travel in nx
+// beside it.  On return X holds the columns, at their own places.
+__device__ int jacobi_regs_f32(int m, float2 *X, float2 *ex, float *nx, float tol, int max_sweeps, int *s_flag,
+                               float *s_off) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int mm = m + (m & 1), np = mm / 2;
+    const bool mine = warp < np;
+    const float tol2 = tol * tol;
+    const bool r0 = lane < m, r1 = lane + 32 < m;
+    // slot t (top, t < np) or np + t (bottom) of the circle; column id of the start: top t = t,
+    // bottom t = mm - 1 - t
+    int ip = warp, iq = mm - 1 - warp;
+    float2 p0 = make_float2(0.f, 0.f), p1 = p0, q0 = p0, q1 = p0;
+    if (mine) {
+        if (lane < m) p0 = X[(size_t)ip * m + lane];
+        if (r1) p1 = X[(size_t)ip * m + lane + 32];
+        if (iq < m) {
+            if (lane < m) q0 = X[(size_t)iq * m + lane];
+            if (r1) q1 = X[(size_t)iq * m + lane + 32];
+        }
+    }
+    // hand on: top t -> top t + 1 (top 0 stays, the last one goes to the bottom), bottom t -> bottom
+    // t - 1 (bottom 0 to top 1); nx: (norm, id) of every slot, two buffers
+    const int tp = warp == 0 ? 0 : warp + 1 < np ? warp + 1 : 2 * np - 1;
+    const int tq = warp == 0 ? (np > 1 ? 1 : np) : np + warp - 1;
+    const int wp = tp * m + lane, wq = tq * m + lane, rp = warp * m + lane, rq = (np + warp) * m + lane;
+    float2 *e = ex, *e2 = ex + mm * m, *en = (float2 *)nx, *en2 = en + mm;
+    int sweep = 0;
+    for (; sweep < max_sweeps; ++sweep) {
+        // column norms, refreshed every sweep
+        float a = warp_sum(p0.x * p0.x + p0.y * p0.y + p1.x * p1.x + p1.y * p1.y);
+        float b = warp_sum(q0.x * q0.x + q0.y * q0.y + q1.x * q1.x + q1.y * q1.y);
+        if (tid == 0) { *s_flag = 0; *s_off = 0.f; }
+        __syncthreads();
+        float wmax = 0.f;                           // largest squared relative off-diagonal this warp saw
+        for (int round = 0; round < mm - 1; ++round) {
+            if (mine) {
+                if (max(ip, iq) < m) {
+                    // gamma = <p, q>: the two sums share one butterfly (lower half re, upper half im)
+                    float gr = p0.x * q0.x + p0.y * q0.y + p1.x * q1.x + p1.y * q1.y;
+                    float gi = p0.x * q0.y - p0.y * q0.x + p1.x * q1.y - p1.y * q1.x;
+                    const bool up = lane & 16;
+                    float v = (up ? gi : gr) + __shfl_xor_sync(0xffffffffu, up ? gr : gi, 16);
+#pragma unroll
+                    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                    const float w = __shfl_xor_sync(0xffffffffu, v, 16);
+                    gr = up ? w : v;
+                    gi = up ? v : w;
+                    const float g2 = fmaf(gr, gr, gi * gi), ab = a * b;
+                    if (g2 > tol2 * ab) {   // |gamma| / sqrt(a b) > tol
+                        wmax = fmaxf(wmax, __fdividef(g2, ab));
+                        // tangent t = sign(d) |gamma| / (|d| + sqrt(d^2 + |gamma|^2)), d = (b - a) / 2; the
+                        // rotation (P, Q) <- (c P - s w Q, c Q + s conj(w) P), w = conj(gamma) / |gamma|
+                        const float ig = rsqrt_nr(g2), ag = g2 * ig, d = 0.5f * (b - a);
+                        const float x = fmaf(d, d, g2), t = __fdividef(copysignf(ag, d), fmaf(x, rsqrtf(x), fabsf(d)));
+                        const float c = rsqrt_nr(fmaf(t, t, 1.f)), si = c * t * ig, sx = si * gr, sy = -si * gi;
+                        auto rot = [&](float2 &p, float2 &q) {
+                            const float2 o = p;
+                            p.x = fmaf(-sx, q.x, fmaf(sy, q.y, c * o.x));
+                            p.y = fmaf(-sx, q.y, fmaf(-sy, q.x, c * o.y));
+                            q.x = fmaf(sx, o.x, fmaf(sy, o.y, c * q.x));
+                            q.y = fmaf(sx, o.y, fmaf(-sy, o.x, c * q.y));
+                        };
+                        rot(p0, q0);
+                        rot(p1, q1);
+                        a = fmaf(-t, ag, a);
+                        b = fmaf(t, ag, b);
+                    }
+                }
+                if (r0) { e[wp] = p0; e[wq] = q0; }
+                if (r1) { e[wp + 32] = p1; e[wq + 32] = q1; }
+                if (lane == 0) {
+                    en[tp] = make_float2(a, __int_as_float(ip));
+                    en[tq] = make_float2(b, __int_as_float(iq));
+                }
+            }
+            __syncthreads();
+            if (mine) {
+                if (r0) { p0 = e[rp]; q0 = e[rq]; }
+                if (r1) { p1 = e[rp + 32]; q1 = e[rq + 32]; }
+                const float2 np_ = en[warp], nq_ = en[np + warp];
+                a = np_.x; ip = __float_as_int(np_.y);
+                b = nq_.x; iq = __float_as_int(nq_.y);
+            }
+            float2 *sw = e; e = e2; e2 = sw;
+            sw = en; en = en2; en2 = sw;
+        }
+        wmax = sqrtf(wmax);
+        if (lane == 0 && wmax > 0.f) {
+            *s_flag = 1;
+            atomicMax((int *)s_off, __float_as_int(wmax));
+        }
+        __syncthreads();
+        if (!*s_flag) break;
+        const float d = *s_off;   // quadratic convergence, as in jacobi_sweeps_f32
+        __syncthreads();
+        if (d * d < tol * 1e-2f) { ++sweep; break; }
+    }
+    if (mine) {
+        if (ip < m) {
+            if (lane < m) X[(size_t)ip * m + lane] = p0;
+            if (r1) X[(size_t)ip * m + lane + 32] = p1;
+        }
+        if (iq < m) {
+            if (lane < m) X[(size_t)iq * m + lane] = q0;
+            if (r1) X[(size_t)iq * m + lane + 32] = q1;
+        }
+    }
+    __syncthreads();
+    return sweep + 1;
+}
+
 // Exact float product as a double-float (FMA two-product).
 __device__ __forceinline__ dfr df_prod(float a, float b) {
     const float p = a * b;
@@ -3197,16 +3339,25 @@ __device__ __forceinline__ dfc to_dfc(double2 a) {
     return c;
 }
 
-// Columns P, Q (length len) <- (c P - s w Q, s P + c w Q), w = wr + i wi.
-__device__ __forceinline__ void rotate_df(dfc *P, dfc *Q, int len, int lane, dfr c, dfr s, dfr wr, dfr wi) {
+// Columns P, Q (length len) <- (c P - g Q, c Q + conj(g) P), g = gx + i gy, c^2 + |g|^2 = 1: each new
+// component is one product and two fused multiply-adds, unnormalised until its end (a quarter of
+// the polish went on normalised products of a phase, c and s in turn).
+__device__ __forceinline__ dfr df_mul_raw(dfr a, dfr b) {
+    const float p = a.hi * b.hi;
+    return dfr(p, fmaf(a.hi, b.lo, fmaf(a.lo, b.hi, fmaf(a.hi, b.hi, -p))));
+}
+__device__ __forceinline__ void rotate_df(dfc *P, dfc *Q, int len, int lane, dfr c, dfr gx, dfr gy) {
     for (int r = lane; r < len; r += 32) {
-        const dfc ap = P[r], q0 = Q[r];
-        const dfr qx = q0.x * wr - q0.y * wi, qy = q0.x * wi + q0.y * wr;
+        const dfc p = P[r], q = Q[r];
+        dfr px = rfma(gy, q.y, rfma(-gx, q.x, df_mul_raw(c, p.x)));
+        dfr py = rfma(-gy, q.x, rfma(-gx, q.y, df_mul_raw(c, p.y)));
+        dfr qx = rfma(gy, p.y, rfma(gx, p.x, df_mul_raw(c, q.x)));
+        dfr qy = rfma(-gy, p.x, rfma(gx, p.y, df_mul_raw(c, q.y)));
         dfc np_, nq_;
-        np_.x = c * ap.x - s * qx;
-        np_.y = c * ap.y - s * qy;
-        nq_.x = s * ap.x + c * qx;
-        nq_.y = s * ap.y + c * qy;
+        np_.x = df_renorm(px.hi, px.lo);
+        np_.y = df_renorm(py.hi, py.lo);
+        nq_.x = df_renorm(qx.hi, qx.lo);
+        nq_.y = df_renorm(qy.hi, qy.lo);
         P[r] = np_;
         Q[r] = nq_;
     }
@@ -3388,8 +3539,22 @@ __device__ int jacobi_polish_df(int m, dfc *A, dfc *V, int ldv, dfr *nrm, float 
                     gi = rfma(ap.x, aq.y, gi);
                     gi = rfma(-ap.y, aq.x, gi);
                 }
-                gr = warp_sum(df_renorm(gr.hi, gr.lo));   // identical in every lane: the two-sum is symmetric
-                gi = warp_sum(df_renorm(gi.hi, gi.lo));
+                // the two sums share one butterfly (lower half re, upper half im); identical in every lane of a
+                // half, and so in every lane after the exchange: the two-sum is symmetric
+                {
+                    const bool up = lane & 16;
+                    gr = df_renorm(gr.hi, gr.lo);
+                    gi = df_renorm(gi.hi, gi.lo);
+                    const dfr give = up ? gr : gi;
+                    dfr v = (up ? gi : gr) + dfr(__shfl_xor_sync(0xffffffffu, give.hi, 16),
+                                                 __shfl_xor_sync(0xffffffffu, give.lo, 16));
+#pragma unroll
+                    for (int o = 8; o > 0; o >>= 1)
+                        v = v + dfr(__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o));
+                    const dfr w(__shfl_xor_sync(0xffffffffu, v.hi, 16), __shfl_xor_sync(0xffffffffu, v.lo, 16));
+                    gr = up ? w : v;
+                    gi = up ? v : w;
+                }
                 const dfr a = nrm[p], b = nrm[q];
                 float t, ag, gx, gy, igs;
                 if (!polish_params(gr, gi, a, b, tol, t, ag, gx, gy, igs)) continue;
@@ -3403,8 +3568,9 @@ __device__ int jacobi_polish_df(int m, dfc *A, dfc *V, int ldv, dfr *nrm, float 
                     const dfr s = c * dfr(t, 0.f);
                     const dfr ig = df_rsqrt(df_prod(gx, gx) + df_prod(gy, gy));
                     const dfr wr = dfr(gx, 0.f) * ig, wi = dfr(-gy, 0.f) * ig;
-                    rotate_df(Ap, Aq, rows, lane, c, s, wr, wi);
-                    rotate_df(V + (size_t)p * ldv, V + (size_t)q * ldv, m, lane, c, s, wr, wi);
+                    const dfr sx = s * wr, sy = s * wi;
+                    rotate_df(Ap, Aq, rows, lane, c, sx, sy);
+                    rotate_df(V + (size_t)p * ldv, V + (size_t)q * ldv, m, lane, c, sx, sy);
                 }
                 if (lane == 0) {
                     const dfr tg = df_prod(t, ag);
@@ -3461,7 +3627,7 @@ __global__ void __launch_bounds__(1024) k_svd(int m, int k, const double2 *__res
     __shared__ float s_off;
     __shared__ unsigned char small_col[168];
     __shared__ int s_emax, s_bad, flag_list[168], perm[168];
-    __shared__ float2 s_c;
+    __shared__ __align__(8) float reg_nx[4 * 64];   // jacobi_regs_f32: norms and ids, two buffers
     // H scaled by the power of two that brings its largest entry into [1, 2): exact, and it
     // keeps the FP32 phase clear of overflow and underflow whatever the operator's scale
     if (tid == 0) s_emax = 0;
@@ -3487,15 +3653,22 @@ __global__ void __launch_bounds__(1024) k_svd(int m, int k, const double2 *__res
     // redone as Jacobi on H accumulating V.
     const float tol32 = 4.0f * 1.1920929e-7f * m;
     const unsigned short *tab32 = (const unsigned short *)Vd;
-    qrcp_f32(m, A32, perm, nrm32, &s_c);
+    if (rows <= 64) qrcp_f32<2>(m, A32, perm, nrm32, (float *)nrmd);
+    else qrcp_f32<6>(m, A32, perm, nrm32, (float *)nrmd);
     float2 *X = V32;                        // m x m, leading dimension m
     for (int e = tid; e < m * m; e += nt) { // X[i][j] = conj(R[j][i]), lower triangular
         const int i = e % m, j = e / m;
-        const float2 r = A32[(size_t)i * rows + j];
+        const float2 r = A32[(size_t)perm[i] * rows + j];
         X[e] = i >= j ? make_float2(r.x, -r.y) : make_float2(0.f, 0.f);
     }
     __syncthreads();
-    int s32 = jacobi_sweeps_f32(m, m, X, nullptr, nrm32, tol32, 40, &s_flag, &s_off, tab32);
+    // the columns in registers where a warp has a pair of its own and two rows a lane hold them (the
+    // exchange buffers take Ad's place, free until phase 2)
+    int s32;
+    if (m <= 64 && m >= 16 && (m + 1) / 2 <= (nt >> 5))
+        s32 = jacobi_regs_f32(m, X, (float2 *)Ad, reg_nx, tol32, 40, &s_flag, &s_off);
+    else
+        s32 = jacobi_sweeps_f32(m, m, X, nullptr, nrm32, tol32, 40, &s_flag, &s_off, tab32);
     {
         const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
         for (int c = warp; c < m; c += nwarps) {
@@ -3602,16 +3775,16 @@ __global__ void __launch_bounds__(1024) k_svd(int m, int k, const double2 *__res
     dfc *T = Sc;                            // m x m, leading dimension m
     for (int e = tid; e < m * m; e += nt) {
         const int i = e % m, j = e / m;     // T[i][j] = sum_l V[i][l] F[l][j]
-        dfr sx(0.f, 0.f), sy(0.f, 0.f);
+        dfr sx(0.f, 0.f), sy(0.f, 0.f);     // unnormalised chains, canonical at the end
         for (int l = 0; l < m; ++l) {
             const dfc v = Vd[(size_t)l * ldv + i], f = E[(size_t)j * m + l];
-            sx = fma(dfr(v.x.hi, 0.f), f.x, sx);
-            sx = fma(dfr(-v.y.hi, 0.f), f.y, sx);
-            sy = fma(dfr(v.x.hi, 0.f), f.y, sy);
-            sy = fma(dfr(v.y.hi, 0.f), f.x, sy);
+            sx = rfma(dfr(v.x.hi, 0.f), f.x, sx);
+            sx = rfma(dfr(-v.y.hi, 0.f), f.y, sx);
+            sy = rfma(dfr(v.x.hi, 0.f), f.y, sy);
+            sy = rfma(dfr(v.y.hi, 0.f), f.x, sy);
         }
-        T[e].x = sx;
-        T[e].y = sy;
+        T[e].x = df_renorm(sx.hi, sx.lo);
+        T[e].y = df_renorm(sy.hi, sy.lo);
     }
     __syncthreads();
     for (int e = tid; e < m * m; e += nt) {
@@ -3624,17 +3797,20 @@ __global__ void __launch_bounds__(1024) k_svd(int m, int k, const double2 *__res
     for (int i = tid; i < rows * m; i += nt) Hd[i] = to_dfc(make_double2(H[i].x * sc, H[i].y * sc));
     __syncthreads();
     for (int e = tid; e < rows * m; e += nt) {
-        const int r = e % rows, c = e / rows;   // A[r][c] = sum_p H[r][p] V[p][c]
+        // A[r][c] = sum_p H[r][p] V[p][c]; unnormalised chains, canonical at the end
+        const int r = e % rows, c = e / rows;
         dfr sx(0.f, 0.f), sy(0.f, 0.f);
         for (int p = 0; p < m; ++p) {
             const dfc h = Hd[(size_t)p * rows + r], v = Vd[(size_t)c * ldv + p];
-            sx = fma(h.x, v.x, sx);
-            sx = fma(-h.y, v.y, sx);
-            sy = fma(h.x, v.y, sy);
-            sy = fma(h.y, v.x, sy);
+            sx = rfma(h.x, v.x, sx);
+            sx = rfma(-h.y, v.y, sx);
+            sy = rfma(h.x, v.y, sy);
+            sy = rfma(h.y, v.x, sy);
         }
-        Ad[e].x = sx;
-        Ad[e].y = sy;
+        dfc a;
+        a.x = df_renorm(sx.hi, sx.lo);
+        a.y = df_renorm(sy.hi, sy.lo);
+        Ad[e] = a;
     }
     __syncthreads();
     // 3. double-float polish of the k smallest.  Sc (H no longer needed) takes the packed pair
@@ -4336,6 +4512,16 @@ __global__ void __launch_bounds__(1024) k_cholqr(int k, double2 *__restrict__ gr
             }
         hd[(size_t)x * ldh + y] = y > x ? zero : make_double2(ldexp(h.x, hx), ldexp(h.y, hx));
     }
+}
+
+// See launch_unit_coordinates.
+__global__ void k_unit_coordinates(int m, int kk, const double2 *__restrict__ coef0, double2 *__restrict__ g0,
+                                   size_t strideC, const int *__restrict__ act, const SysState *__restrict__ state) {
+    const int s = act[blockIdx.x];
+    const double2 *coef = coef0 + (size_t)s * strideC;
+    double2 *g = g0 + (size_t)s * strideC;
+    for (int p = threadIdx.x; p <= m; p += blockDim.x)
+        g[p] = p < kk ? coef[p] : make_double2(p > kk ? 0.0 : kk > 0 ? sqrt(state[s].nrm2) : 1.0, 0.0);
 }
 
 __global__ void k_broadcast_hdef(int m, int kk, const double2 *__restrict__ Hd, double2 *__restrict__ H0, size_t strideH,
@@ -5302,13 +5488,19 @@ void launch_znormalise(int n, int k, const typename CT<R>::t *Znew, const double
     k_znormalise<R><<<grid2(stream_grid<R>(n, k), k), NT, 0, st>>>(n, Znew, znorm2, Z);
 }
 
+void launch_unit_coordinates(int m, int kk, const double2 *coef, double2 *g, size_t strideC, const int *act, int nsys,
+                             const SysState *state, cudaStream_t st) {
+    Launch L_(KC_OTHER, 0.0, st, 1);
+    k_unit_coordinates<<<nsys, 64, 0, st>>>(m, kk, coef, g, strideC, act, state);
+}
+
 void launch_ls(int m, const double2 *H, size_t strideH, const double2 *g, double2 *y, double2 *t, size_t strideC,
                const int *act, int nsys, cudaStream_t st) {
     if (nsys <= 0) return;
     Launch L_(KC_LS, (double)sizeof(double2) * nsys * (m + 1.0) * m, st, 1);
-    size_t smem = sizeof(double2) * ((size_t)m * (m + 3) / 2 + (m + 1) + m + m) + sizeof(double) * (m + 1);
+    size_t smem = sizeof(double2) * ((size_t)m * (m + 3) / 2 + (m + 1) + 3 * m) + sizeof(double) * m;
     allow_smem(k_ls, smem);
-    k_ls<<<nsys, 128, smem, st>>>(m, H, strideH, g, y, t, strideC, act);
+    k_ls<<<nsys, ((m + 1 + 31) / 32) * 32, smem, st>>>(m, H, strideH, g, y, t, strideC, act);
 }
 
 size_t svd_smem_bytes(int m) { return svd_work_bytes(m); }

@@ -355,6 +355,11 @@ template <class R>
 void launch_znormalise(int n, int k, const typename CT<R>::t *Znew, const double *znorm2, typename CT<R>::t *Z,
                        cudaStream_t st);
 
+// The coordinates g of a refined cycle's unit residual r in [W V] when v_0 comes from r itself: r = W a + nrm v_0
+// with a = W^H r (coef, kk of them) and nrm the norm of the projected r (state nrm2, just reduced), so
+// g = (a, nrm, 0, ..., 0); with kk = 0, v_0 = r.
+void launch_unit_coordinates(int m, int kk, const double2 *coef, double2 *g, size_t strideC, const int *act, int nsys,
+                             const SysState *state, cudaStream_t st);
 // Batched least squares min ||H_s y - g_s|| (FP64 Givens), t_s = H_s y_s.
 void launch_ls(int m, const double2 *H, size_t strideH, const double2 *g, double2 *y, double2 *t, size_t strideC,
                const int *act, int nsys, cudaStream_t st);
