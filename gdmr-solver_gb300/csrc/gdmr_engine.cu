@@ -266,12 +266,21 @@ int sell_from_csr(DeviceSell &out, int n, const int *rowptr, const int *colidx, 
     // coefficient planes, duplicates of one column added in CSR order as for uniform slices
     const size_t gsz = gx ? (size_t)np * n : 0;
     std::vector<double> gre(gsz, 0.0), gim(gsz, 0.0);
+    // every entry of plane e equal to its first, and how many there are; a second entry of one place rules the
+    // matrix out (constant planes, below)
+    struct Plane { double re = 0, im = 0; long count = 0; } first[SELL_PATTERN];
+    bool same = gx > 0;
     if (gx)
         for (int r = 0; r < n; ++r)
             for (int q = rowptr[r]; q < rowptr[r + 1]; ++q) {
                 const size_t e = (size_t)(std::find(pat.begin(), pat.end(), colidx[q] - r) - pat.begin());
-                gre[e * n + r] += vals_ri[2 * (size_t)q];
-                gim[e * n + r] += vals_ri[2 * (size_t)q + 1];
+                const double re = vals_ri[2 * (size_t)q], im = vals_ri[2 * (size_t)q + 1];
+                double &a = gre[e * n + r], &b = gim[e * n + r];
+                Plane &f = first[e];
+                if (f.count++ == 0) { f.re = re; f.im = im; }
+                same = same && re == f.re && im == f.im && a == 0.0 && b == 0.0;
+                a += re;
+                b += im;
             }
     DeviceSell d;
     // a failed allocation or copy frees what was already allocated
@@ -337,24 +346,13 @@ int sell_from_csr(DeviceSell &out, int n, const int *rowptr, const int *colidx, 
             if (real) d.greal |= 1u << e;
         }
         // constant planes: one value wherever the neighbour lies on the grid
-        bool same = true;
-        const long plane = (long)gx * gy;
-        const int p0 = gz > 1 ? 0 : 1;
-        for (int e = 0; same && e < np; ++e) {
-            const int p = e + p0;                       // 7-plane index: -P, -Q, -1, 0, +1, +Q, +P
-            bool any = false;
-            double re = 0, im = 0;
-            for (int r = 0; same && r < n; ++r) {
-                const int x = r % gx, y = (int)((r / gx) % gy), z = (int)(r / plane);
-                if ((p == 0 && z == 0) || (p == 1 && y == 0) || (p == 2 && x == 0) || (p == 4 && x + 1 == gx) ||
-                    (p == 5 && y + 1 == gy) || (p == 6 && z + 1 == gz))
-                    continue;
-                const double a = gre[(size_t)e * n + r], b = gim[(size_t)e * n + r];
-                if (!any) { re = a; im = b; any = true; }
-                same = a == re && b == im;
-            }
-            d.gconst.a[p] = make_double2(re, im);
-            if (im == 0.0) d.gconst.real |= 1u << p;
+        const int p0 = gz > 1 ? 0 : 1;                  // 7-plane index: -P, -Q, -1, 0, +1, +Q, +P
+        for (int e = 0; e < np; ++e) {
+            const int p = e + p0;
+            const long cut = p == 0 || p == 6 ? gz : p == 1 || p == 5 ? gy : p == 2 || p == 4 ? gx : 0;
+            same = same && first[e].count == (cut ? (long)n - n / cut : (long)n);
+            d.gconst.a[p] = make_double2(first[e].re, first[e].im);
+            if (first[e].im == 0.0) d.gconst.real |= 1u << p;
         }
         d.gconst.valid = same;
         // one precision at a time, each host copy released after its upload
