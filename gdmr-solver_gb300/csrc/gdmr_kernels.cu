@@ -4,6 +4,7 @@
 #include <type_traits>
 
 #include <math.h>
+#include <stddef.h>
 
 #include <algorithm>
 #include <atomic>
@@ -3196,47 +3197,120 @@ __device__ int jacobi_sweeps_f32(int m, int rows, float2 *A, float2 *V, float *n
     return sweep + 1;
 }
 
-// jacobi_sweeps_f32 without V for rows = m <= 64 and a warp a pair: each warp keeps its two columns in
-// registers, two rows a lane, and a round hands them on through shared memory along the circle (the top
-// row to the right, the bottom row to the left), double-buffered in `ex` (2 x mm columns of m float2, mm = m
-// rounded up to even).  One barrier a round, the columns read and written once (the in-place form reads them twice:
-// 2100 clocks a round at m = 48, bound by its instructions).  A column's squared norm and id travel in nx
-// beside it.  On return X holds the columns, at their own places.
-__device__ int jacobi_regs_f32(int m, float2 *X, float2 *ex, float *nx, float tol, int max_sweeps, int *s_flag,
-                               float *s_off) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int mm = m + (m & 1), np = mm / 2;
-    const bool mine = warp < np;
+// ---- distributed shared memory of a thread-block cluster
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ unsigned cluster_size() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;\n" : "=r"(r));
+    return r;
+}
+// Barrier over the cluster's threads, shared-memory writes (remote ones too) ordered by it.
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// The shared::cluster address of `p` (this CTA's shared memory) in CTA `rank`.
+__device__ __forceinline__ unsigned map_shared(const void *p, unsigned rank) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_remote(unsigned a, float2 v) {
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
+}
+__device__ __forceinline__ void st_remote(unsigned a, dfc v) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"r"(a), "f"(v.x.hi), "f"(v.x.lo), "f"(v.y.hi),
+                 "f"(v.y.lo)
+                 : "memory");
+}
+__device__ __forceinline__ void ld_remote(unsigned a, float2 &v) {
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void ld_remote(unsigned a, dfc &v) {
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+                 : "=f"(v.x.hi), "=f"(v.x.lo), "=f"(v.y.hi), "=f"(v.y.lo) : "r"(a) : "memory");
+}
+__device__ __forceinline__ int ld_remote_int(unsigned a) {
+    int v;
+    asm volatile("ld.shared::cluster.s32 %0, [%1];\n" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void max_remote(unsigned a, int v) {
+    asm volatile("red.relaxed.cluster.shared::cluster.max.s32 [%0], %1;\n" ::"r"(a), "r"(v) : "memory");
+}
+
+// One-sided Jacobi over a cluster.  A round's pairs are independent, and in one CTA their instructions, not
+// their latency, fill the round (2000 clocks in FP32, 5500 in double-float at m = 48, 24 pairs): so the pairs
+// are dealt to the cluster's CTAs, wpc warps each, every warp keeping its two columns in registers, two rows a
+// lane (at most 64 rows).  A round ends by handing the columns on along the circle (the top row to the right,
+// the bottom row to the left) through the receiving CTA's shared memory, double-buffered, with one cluster
+// barrier.  Slot w of the circle (the pair of warp w of the cluster) starts with columns w and mm - 1 - w, and
+// after a sweep's mm - 1 rounds every column is back.
+struct CircleSlot {
+    int np, wpc, w;          // pairs, pairs a CTA, this warp's pair
+    unsigned rank;
+    bool mine;
+    int to_p, to_q;          // exchange slots (in their CTAs) of the columns handed on
+    unsigned cta_p, cta_q;
+};
+__device__ __forceinline__ CircleSlot circle_slot(int m) {
+    CircleSlot c;
+    const int mm = m + (m & 1), warp = threadIdx.x >> 5, nc = (int)cluster_size();
+    c.np = mm / 2;
+    c.wpc = (c.np + nc - 1) / nc;
+    c.rank = cluster_rank();
+    c.w = (int)c.rank * c.wpc + warp;
+    c.mine = warp < c.wpc && c.w < c.np;
+    // top t -> top t + 1 (top 0 stays, the last one goes to the bottom), bottom t -> bottom t - 1
+    // (bottom 0 to top 1)
+    const bool p_top = c.w == 0 || c.w + 1 < c.np, q_top = c.w == 0 && c.np > 1;
+    const int wp = c.w == 0 ? 0 : c.w + 1 < c.np ? c.w + 1 : c.np - 1, wq = c.w == 0 ? (c.np > 1 ? 1 : 0) : c.w - 1;
+    c.cta_p = (unsigned)(wp / c.wpc);
+    c.cta_q = (unsigned)(wq / c.wpc);
+    c.to_p = wp % c.wpc + (p_top ? 0 : c.wpc);
+    c.to_q = wq % c.wpc + (q_top ? 0 : c.wpc);
+    return c;
+}
+// Loop control of a phase, in CTA 0's shared memory.
+struct ClusterFlags {
+    int off;      // largest off-diagonal of the sweep (float bits; 0: no rotation)
+    int done;     // CTA 0's verdict
+};
+
+// FP32 sweeps on CTA 0's X (m x m, m <= 64, no accumulation); ex: exchange buffers in every CTA's shared memory at
+// the same place, 4 wpc (m + 1) float2.  Every thread of the cluster calls it; returns the sweeps + 1.
+__device__ int jacobi_cluster_f32(int m, float2 *X, float2 *ex, float tol, int max_sweeps, ClusterFlags *fl) {
+    const int lane = threadIdx.x & 31, mm = m + (m & 1);
+    const CircleSlot cs = circle_slot(m);
+    const int warp = threadIdx.x >> 5, stride = m + 1;       // a column and its (norm, id)
     const float tol2 = tol * tol;
     const bool r0 = lane < m, r1 = lane + 32 < m;
-    // slot t (top, t < np) or np + t (bottom) of the circle; column id of the start: top t = t,
-    // bottom t = mm - 1 - t
-    int ip = warp, iq = mm - 1 - warp;
+    const unsigned x0 = map_shared(X, 0), f0 = map_shared(fl, 0);
+    const unsigned ep = map_shared(ex + cs.to_p * stride, cs.cta_p), eq = map_shared(ex + cs.to_q * stride, cs.cta_q);
+    const unsigned half = (unsigned)(2 * cs.wpc * stride * sizeof(float2));
+    const float2 *my = ex + warp * stride;
+    cluster_barrier();                                        // CTA 0's X is complete
+    int ip = cs.w, iq = mm - 1 - cs.w;
     float2 p0 = make_float2(0.f, 0.f), p1 = p0, q0 = p0, q1 = p0;
-    if (mine) {
-        if (lane < m) p0 = X[(size_t)ip * m + lane];
-        if (r1) p1 = X[(size_t)ip * m + lane + 32];
-        if (iq < m) {
-            if (lane < m) q0 = X[(size_t)iq * m + lane];
-            if (r1) q1 = X[(size_t)iq * m + lane + 32];
-        }
+    if (cs.mine) {
+        if (r0) ld_remote(x0 + (ip * m + lane) * 8, p0);
+        if (r1) ld_remote(x0 + (ip * m + lane + 32) * 8, p1);
+        if (iq < m && r0) ld_remote(x0 + (iq * m + lane) * 8, q0);
+        if (iq < m && r1) ld_remote(x0 + (iq * m + lane + 32) * 8, q1);
     }
-    // hand on: top t -> top t + 1 (top 0 stays, the last one goes to the bottom), bottom t -> bottom
-    // t - 1 (bottom 0 to top 1); nx: (norm, id) of every slot, two buffers
-    const int tp = warp == 0 ? 0 : warp + 1 < np ? warp + 1 : 2 * np - 1;
-    const int tq = warp == 0 ? (np > 1 ? 1 : np) : np + warp - 1;
-    const int wp = tp * m + lane, wq = tq * m + lane, rp = warp * m + lane, rq = (np + warp) * m + lane;
-    float2 *e = ex, *e2 = ex + mm * m, *en = (float2 *)nx, *en2 = en + mm;
     int sweep = 0;
+    unsigned par = 0;
     for (; sweep < max_sweeps; ++sweep) {
         // column norms, refreshed every sweep
         float a = warp_sum(p0.x * p0.x + p0.y * p0.y + p1.x * p1.x + p1.y * p1.y);
         float b = warp_sum(q0.x * q0.x + q0.y * q0.y + q1.x * q1.x + q1.y * q1.y);
-        if (tid == 0) { *s_flag = 0; *s_off = 0.f; }
-        __syncthreads();
-        float wmax = 0.f;                           // largest squared relative off-diagonal this warp saw
-        for (int round = 0; round < mm - 1; ++round) {
-            if (mine) {
+        if (cs.rank == 0 && threadIdx.x == 0) fl->off = 0;   // read again after the sweep's barriers
+        float wmax = 0.f;                                     // largest squared relative off-diagonal
+        for (int round = 0; round < mm - 1; ++round, par ^= 1) {
+            if (cs.mine) {
                 if (max(ip, iq) < m) {
                     // gamma = <p, q>: the two sums share one butterfly (lower half re, upper half im)
                     float gr = p0.x * q0.x + p0.y * q0.y + p1.x * q1.x + p1.y * q1.y;
@@ -3269,46 +3343,40 @@ __device__ int jacobi_regs_f32(int m, float2 *X, float2 *ex, float *nx, float to
                         b = fmaf(t, ag, b);
                     }
                 }
-                if (r0) { e[wp] = p0; e[wq] = q0; }
-                if (r1) { e[wp + 32] = p1; e[wq + 32] = q1; }
+                const unsigned tp = ep + par * half, tq = eq + par * half;
+                if (r0) { st_remote(tp + lane * 8, p0); st_remote(tq + lane * 8, q0); }
+                if (r1) { st_remote(tp + (lane + 32) * 8, p1); st_remote(tq + (lane + 32) * 8, q1); }
                 if (lane == 0) {
-                    en[tp] = make_float2(a, __int_as_float(ip));
-                    en[tq] = make_float2(b, __int_as_float(iq));
+                    st_remote(tp + m * 8, make_float2(a, __int_as_float(ip)));
+                    st_remote(tq + m * 8, make_float2(b, __int_as_float(iq)));
                 }
             }
-            __syncthreads();
-            if (mine) {
-                if (r0) { p0 = e[rp]; q0 = e[rq]; }
-                if (r1) { p1 = e[rp + 32]; q1 = e[rq + 32]; }
-                const float2 np_ = en[warp], nq_ = en[np + warp];
+            cluster_barrier();
+            if (cs.mine) {
+                const float2 *e = my + par * 2 * cs.wpc * stride, *f = e + cs.wpc * stride;
+                if (r0) { p0 = e[lane]; q0 = f[lane]; }
+                if (r1) { p1 = e[lane + 32]; q1 = f[lane + 32]; }
+                const float2 np_ = e[m], nq_ = f[m];
                 a = np_.x; ip = __float_as_int(np_.y);
                 b = nq_.x; iq = __float_as_int(nq_.y);
             }
-            float2 *sw = e; e = e2; e2 = sw;
-            sw = en; en = en2; en2 = sw;
         }
-        wmax = sqrtf(wmax);
-        if (lane == 0 && wmax > 0.f) {
-            *s_flag = 1;
-            atomicMax((int *)s_off, __float_as_int(wmax));
-        }
-        __syncthreads();
-        if (!*s_flag) break;
-        const float d = *s_off;   // quadratic convergence, as in jacobi_sweeps_f32
-        __syncthreads();
-        if (d * d < tol * 1e-2f) { ++sweep; break; }
+        if (cs.mine && lane == 0 && wmax > 0.f) max_remote(f0, __float_as_int(wmax));
+        cluster_barrier();
+        const float d2 = __int_as_float(ld_remote_int(f0));   // squared
+        cluster_barrier();                                    // every thread has read it
+        if (!(d2 > 0.f)) break;
+        // quadratic convergence: after a sweep whose largest relative off-diagonal was d, the next is
+        // of order d^2; stop once that is below the tolerance
+        if (d2 < tol * 1e-2f) { ++sweep; break; }
     }
-    if (mine) {
-        if (ip < m) {
-            if (lane < m) X[(size_t)ip * m + lane] = p0;
-            if (r1) X[(size_t)ip * m + lane + 32] = p1;
-        }
-        if (iq < m) {
-            if (lane < m) X[(size_t)iq * m + lane] = q0;
-            if (r1) X[(size_t)iq * m + lane + 32] = q1;
-        }
+    if (cs.mine) {
+        if (r0) st_remote(x0 + (ip * m + lane) * 8, p0);
+        if (r1) st_remote(x0 + (ip * m + lane + 32) * 8, p1);
+        if (iq < m && r0) st_remote(x0 + (iq * m + lane) * 8, q0);
+        if (iq < m && r1) st_remote(x0 + (iq * m + lane + 32) * 8, q1);
     }
-    __syncthreads();
+    cluster_barrier();
     return sweep + 1;
 }
 
@@ -3346,20 +3414,23 @@ __device__ __forceinline__ dfr df_mul_raw(dfr a, dfr b) {
     const float p = a.hi * b.hi;
     return dfr(p, fmaf(a.hi, b.lo, fmaf(a.lo, b.hi, fmaf(a.hi, b.hi, -p))));
 }
+__device__ __forceinline__ void rotate_df_one(dfc &P, dfc &Q, dfr c, dfr gx, dfr gy) {
+    const dfc p = P, q = Q;
+    const dfr px = rfma(gy, q.y, rfma(-gx, q.x, df_mul_raw(c, p.x)));
+    const dfr py = rfma(-gy, q.x, rfma(-gx, q.y, df_mul_raw(c, p.y)));
+    const dfr qx = rfma(gy, p.y, rfma(gx, p.x, df_mul_raw(c, q.x)));
+    const dfr qy = rfma(-gy, p.x, rfma(gx, p.y, df_mul_raw(c, q.y)));
+    P.x = df_renorm(px.hi, px.lo);
+    P.y = df_renorm(py.hi, py.lo);
+    Q.x = df_renorm(qx.hi, qx.lo);
+    Q.y = df_renorm(qy.hi, qy.lo);
+}
 __device__ __forceinline__ void rotate_df(dfc *P, dfc *Q, int len, int lane, dfr c, dfr gx, dfr gy) {
     for (int r = lane; r < len; r += 32) {
-        const dfc p = P[r], q = Q[r];
-        dfr px = rfma(gy, q.y, rfma(-gx, q.x, df_mul_raw(c, p.x)));
-        dfr py = rfma(-gy, q.x, rfma(-gx, q.y, df_mul_raw(c, p.y)));
-        dfr qx = rfma(gy, p.y, rfma(gx, p.x, df_mul_raw(c, q.x)));
-        dfr qy = rfma(-gy, p.x, rfma(gx, p.y, df_mul_raw(c, q.y)));
-        dfc np_, nq_;
-        np_.x = df_renorm(px.hi, px.lo);
-        np_.y = df_renorm(py.hi, py.lo);
-        nq_.x = df_renorm(qx.hi, qx.lo);
-        nq_.y = df_renorm(qy.hi, qy.lo);
-        P[r] = np_;
-        Q[r] = nq_;
+        dfc p = P[r], q = Q[r];
+        rotate_df_one(p, q, c, gx, gy);
+        P[r] = p;
+        Q[r] = q;
     }
 }
 // a + b for a double-float a and a float b.
@@ -3600,6 +3671,191 @@ __device__ int jacobi_polish_df(int m, dfc *A, dfc *V, int ldv, dfr *nrm, float 
     return sweep + 1;
 }
 
+// jacobi_polish_df over a cluster (see jacobi_cluster_f32), rows = m + 1 <= 64: A and V of CTA 0, whose threads
+// also run polish_small_all between the sweeps, on the columns written back to it.  ex: 4 wpc
+// (2 m + 2) dfc in every CTA's shared memory, beside A and V.  Every thread of the cluster calls it; on
+// CTA 0 the squared norms of the result are in nrm on return, as jacobi_polish_df leaves them.
+__device__ int jacobi_polish_cluster(int m, dfc *A, dfc *V, int ldv, dfr *nrm, float tol, int max_sweeps,
+                                     const unsigned char *small_col, const int *flg, int k, float2 *C, dfc *ex,
+                                     ClusterFlags *fl) {
+    const int rows = m + 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    const int mm = m + (m & 1), stride = rows + m + 1;       // a column of A, of V, (norm, id)
+    const CircleSlot cs = circle_slot(m);
+    __shared__ int s_big;
+    const bool a0 = lane < rows, a1 = lane + 32 < rows, v0 = lane < m, v1 = lane + 32 < m;
+    const unsigned A0 = map_shared(A, 0), V0 = map_shared(V, 0), f0 = map_shared(fl, 0), sc0 = map_shared(small_col, 0);
+    const unsigned ep = map_shared(ex + cs.to_p * stride, cs.cta_p), eq = map_shared(ex + cs.to_q * stride, cs.cta_q);
+    const unsigned half = (unsigned)(2 * cs.wpc * stride * sizeof(dfc));
+    const dfc *my = ex + warp * stride;
+    dfc z;
+    z.x = dfr(0.f, 0.f);
+    z.y = dfr(0.f, 0.f);
+    auto column_norms = [&]() {                               // of CTA 0's A
+        for (int c = warp; c < m; c += nwarps) {
+            dfr a(0.f, 0.f);
+            for (int r = lane; r < rows; r += 32) {
+                const dfc v = A[(size_t)c * rows + r];
+                a = fma(v.x, v.x, a);
+                a = fma(v.y, v.y, a);
+            }
+            a = warp_sum(a);
+            if (lane == 0) nrm[c] = a;
+        }
+    };
+    cluster_barrier();                                        // CTA 0's A, V and flags are complete
+    // the flagged columns as two words (small_col: one byte a column)
+    unsigned lo, hi;
+    {
+        unsigned b0 = 0, b1 = 0;
+        if (lane < m) asm volatile("ld.shared::cluster.u8 %0, [%1];\n" : "=r"(b0) : "r"(sc0 + lane) : "memory");
+        if (lane + 32 < m) asm volatile("ld.shared::cluster.u8 %0, [%1];\n" : "=r"(b1) : "r"(sc0 + lane + 32) : "memory");
+        lo = __ballot_sync(0xffffffffu, b0 != 0);
+        hi = __ballot_sync(0xffffffffu, b1 != 0);
+    }
+    auto flagged = [&](int c) { return ((c < 32 ? lo >> c : hi >> (c - 32)) & 1u) != 0; };
+    int ip = cs.w, iq = mm - 1 - cs.w;
+    dfc pa[2] = {z, z}, pv[2] = {z, z}, qa[2] = {z, z}, qv[2] = {z, z};
+    if (cs.mine) {
+        if (a0) ld_remote(A0 + (ip * rows + lane) * 16, pa[0]);
+        if (a1) ld_remote(A0 + (ip * rows + lane + 32) * 16, pa[1]);
+        if (v0) ld_remote(V0 + (ip * ldv + lane) * 16, pv[0]);
+        if (v1) ld_remote(V0 + (ip * ldv + lane + 32) * 16, pv[1]);
+        if (iq < m) {
+            if (a0) ld_remote(A0 + (iq * rows + lane) * 16, qa[0]);
+            if (a1) ld_remote(A0 + (iq * rows + lane + 32) * 16, qa[1]);
+            if (v0) ld_remote(V0 + (iq * ldv + lane) * 16, qv[0]);
+            if (v1) ld_remote(V0 + (iq * ldv + lane + 32) * 16, qv[1]);
+        }
+    }
+    int sweep = 0;
+    unsigned par = 0;
+    bool fresh = false;                                       // nrm matches CTA 0's A
+    for (; sweep < max_sweeps; ++sweep) {
+        if (sweep > 0) {
+            if (cs.rank == 0) {
+                column_norms();
+                __syncthreads();
+                const bool ok = polish_small_all(m, A, V, ldv, nrm, tol, flg, k, C, &s_big);
+                if (tid == 0) fl->done = ok ? 1 : 0;
+            }
+            cluster_barrier();
+            const int done = ld_remote_int(f0 + (unsigned)offsetof(ClusterFlags, done));
+            cluster_barrier();
+            if (done) {
+                ++sweep;
+                fresh = true;
+                break;
+            }
+        }
+        dfr a(0.f, 0.f), b(0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            a = fma(pa[u].x, pa[u].x, a);
+            a = fma(pa[u].y, pa[u].y, a);
+            b = fma(qa[u].x, qa[u].x, b);
+            b = fma(qa[u].y, qa[u].y, b);
+        }
+        a = warp_sum(a);
+        b = warp_sum(b);
+        if (cs.rank == 0 && tid == 0) fl->off = 0;
+        float wmax = 0.f;
+        for (int round = 0; round < mm - 1; ++round, par ^= 1) {
+            if (cs.mine) {
+                if (max(ip, iq) < m && (flagged(ip) || flagged(iq))) {
+                    dfr gr(0.f, 0.f), gi(0.f, 0.f);
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {             // unnormalised chains, canonical below
+                        gr = rfma(pa[u].x, qa[u].x, gr);
+                        gr = rfma(pa[u].y, qa[u].y, gr);
+                        gi = rfma(pa[u].x, qa[u].y, gi);
+                        gi = rfma(-pa[u].y, qa[u].x, gi);
+                    }
+                    // the two sums share one butterfly (lower half re, upper half im); the two-sum is
+                    // symmetric, so every lane ends with the same values
+                    {
+                        const bool up = lane & 16;
+                        gr = df_renorm(gr.hi, gr.lo);
+                        gi = df_renorm(gi.hi, gi.lo);
+                        const dfr give = up ? gr : gi;
+                        dfr v = (up ? gi : gr) + dfr(__shfl_xor_sync(0xffffffffu, give.hi, 16),
+                                                     __shfl_xor_sync(0xffffffffu, give.lo, 16));
+#pragma unroll
+                        for (int o = 8; o > 0; o >>= 1)
+                            v = v + dfr(__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o));
+                        const dfr w(__shfl_xor_sync(0xffffffffu, v.hi, 16), __shfl_xor_sync(0xffffffffu, v.lo, 16));
+                        gr = up ? w : v;
+                        gi = up ? v : w;
+                    }
+                    float t, ag, gx, gy, igs;
+                    if (polish_params(gr, gi, a, b, tol, t, ag, gx, gy, igs)) {
+                        wmax = fmaxf(wmax, ag * rsqrtf(a.hi) * rsqrtf(b.hi));
+                        const dfr c = df_rsqrt(dfr(1.f, 0.f) + df_prod(t, t));
+                        const dfr sn = c * dfr(t, 0.f);
+                        const dfr ig = df_rsqrt(df_prod(gx, gx) + df_prod(gy, gy));
+                        const dfr sx = sn * (dfr(gx, 0.f) * ig), sy = sn * (dfr(-gy, 0.f) * ig);
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            rotate_df_one(pa[u], qa[u], c, sx, sy);
+                            rotate_df_one(pv[u], qv[u], c, sx, sy);
+                        }
+                        const dfr tg = df_prod(t, ag);
+                        a = a - tg;
+                        b = b + tg;
+                    }
+                }
+                const unsigned tp = ep + par * half, tq = eq + par * half;
+                if (a0) { st_remote(tp + lane * 16, pa[0]); st_remote(tq + lane * 16, qa[0]); }
+                if (a1) { st_remote(tp + (lane + 32) * 16, pa[1]); st_remote(tq + (lane + 32) * 16, qa[1]); }
+                if (v0) { st_remote(tp + (rows + lane) * 16, pv[0]); st_remote(tq + (rows + lane) * 16, qv[0]); }
+                if (v1) { st_remote(tp + (rows + lane + 32) * 16, pv[1]); st_remote(tq + (rows + lane + 32) * 16, qv[1]); }
+                if (lane == 0) {
+                    dfc np_, nq_;
+                    np_.x = a;
+                    np_.y = dfr(__int_as_float(ip), 0.f);
+                    nq_.x = b;
+                    nq_.y = dfr(__int_as_float(iq), 0.f);
+                    st_remote(tp + (rows + m) * 16, np_);
+                    st_remote(tq + (rows + m) * 16, nq_);
+                }
+            }
+            cluster_barrier();
+            if (cs.mine) {
+                const dfc *e = my + par * 2 * cs.wpc * stride, *f = e + cs.wpc * stride;
+                if (a0) { pa[0] = e[lane]; qa[0] = f[lane]; }
+                if (a1) { pa[1] = e[lane + 32]; qa[1] = f[lane + 32]; }
+                if (v0) { pv[0] = e[rows + lane]; qv[0] = f[rows + lane]; }
+                if (v1) { pv[1] = e[rows + lane + 32]; qv[1] = f[rows + lane + 32]; }
+                const dfc np_ = e[rows + m], nq_ = f[rows + m];
+                a = np_.x; ip = __float_as_int(np_.y.hi);
+                b = nq_.x; iq = __float_as_int(nq_.y.hi);
+            }
+        }
+        // the columns back to CTA 0
+        if (cs.mine) {
+            if (a0) st_remote(A0 + (ip * rows + lane) * 16, pa[0]);
+            if (a1) st_remote(A0 + (ip * rows + lane + 32) * 16, pa[1]);
+            if (v0) st_remote(V0 + (ip * ldv + lane) * 16, pv[0]);
+            if (v1) st_remote(V0 + (ip * ldv + lane + 32) * 16, pv[1]);
+            if (iq < m) {
+                if (a0) st_remote(A0 + (iq * rows + lane) * 16, qa[0]);
+                if (a1) st_remote(A0 + (iq * rows + lane + 32) * 16, qa[1]);
+                if (v0) st_remote(V0 + (iq * ldv + lane) * 16, qv[0]);
+                if (v1) st_remote(V0 + (iq * ldv + lane + 32) * 16, qv[1]);
+            }
+            if (lane == 0 && wmax > 0.f) max_remote(f0, __float_as_int(wmax));
+        }
+        cluster_barrier();
+        const float d = __int_as_float(ld_remote_int(f0));
+        cluster_barrier();
+        if (!(d > 0.f)) break;
+        if (d * d < tol * 1e-2f) { ++sweep; break; }
+    }
+    if (!fresh && cs.rank == 0) column_norms();
+    __syncthreads();
+    cluster_barrier();                                        // no CTA leaves while another may address it
+    return sweep + 1;
+}
+
 // Working storage of k_svd, three regions of 16 (m+1) m bytes (shared memory when it fits):
 //   Ad  (m+1) x m double-float complex, A = H V;
 //   Vd  m x m, leading dimension m | 1 (odd, so the column-strided reads of V^H V hit
@@ -3608,14 +3864,18 @@ __device__ int jacobi_polish_df(int m, dfc *A, dfc *V, int ldv, dfr *nrm, float 
 //       double-float (E and F live in Ad until A is formed).
 __host__ __device__ inline size_t svd_work_bytes(int m) { return 3 * sizeof(dfc) * (size_t)(m + 1) * m; }
 
-__global__ void __launch_bounds__(1024) k_svd(int m, int k, const double2 *__restrict__ H0, size_t strideH,
+// Clustered (SVD_CLUSTER_THREADS a CTA) or one CTA (up to 1024).
+constexpr int SVD_CLUSTER_THREADS = 768;
+template <bool clustered>
+__global__ void __launch_bounds__(clustered ? SVD_CLUSTER_THREADS : 1024) k_svd(int m, int k, const double2 *__restrict__ H0, size_t strideH,
                                               const int *__restrict__ lead, double2 *__restrict__ vs,
                                               double *__restrict__ sigma, double2 *__restrict__ gwork, int use_smem,
                                               int *sweeps_out) {
     const double2 *__restrict__ H = H0 + (size_t)(*lead) * strideH;
     extern __shared__ __align__(16) unsigned char svd_sm[];
     const int rows = m + 1, tid = threadIdx.x, nt = blockDim.x, ldv = m | 1;
-    unsigned char *base = use_smem ? svd_sm : (unsigned char *)gwork;
+    unsigned char *base = clustered || use_smem ? svd_sm : (unsigned char *)gwork;
+    dfc *ex = (dfc *)(svd_sm + svd_work_bytes(m));   // exchange buffers of the clustered sweeps
     dfc *Ad = (dfc *)base;
     dfc *Vd = Ad + (size_t)rows * m;
     dfc *Sc = Vd + (size_t)rows * m;
@@ -3627,7 +3887,16 @@ __global__ void __launch_bounds__(1024) k_svd(int m, int k, const double2 *__res
     __shared__ float s_off;
     __shared__ unsigned char small_col[168];
     __shared__ int s_emax, s_bad, flag_list[168], perm[168];
-    __shared__ __align__(8) float reg_nx[4 * 64];   // jacobi_regs_f32: norms and ids, two buffers
+    __shared__ ClusterFlags s_fl;
+    const float tol32 = 4.0f * 1.1920929e-7f * m, toldf = 4.0f * 2.220446e-16f * m;
+    if constexpr (clustered) {
+        if (cluster_rank() != 0) {
+            // the other CTAs take their share of the pairs in the two Jacobi phases
+            jacobi_cluster_f32(m, (float2 *)Sc + (size_t)rows * m, (float2 *)ex, tol32, 40, &s_fl);
+            jacobi_polish_cluster(m, Ad, Vd, ldv, nrmd, toldf, 30, small_col, flag_list, k, nullptr, ex, &s_fl);
+            return;
+        }
+    }
     // H scaled by the power of two that brings its largest entry into [1, 2): exact, and it
     // keeps the FP32 phase clear of overflow and underflow whatever the operator's scale
     if (tid == 0) s_emax = 0;
@@ -3651,7 +3920,6 @@ __global__ void __launch_bounds__(1024) k_svd(int m, int k, const double2 *__res
     // vectors of R scaled by the singular values, and H's are V = P V_R.  Should a column come
     // out too small to normalise (singular values below ~1e-15 of the largest), the phase is
     // redone as Jacobi on H accumulating V.
-    const float tol32 = 4.0f * 1.1920929e-7f * m;
     const unsigned short *tab32 = (const unsigned short *)Vd;
     if (rows <= 64) qrcp_f32<2>(m, A32, perm, nrm32, (float *)nrmd);
     else qrcp_f32<6>(m, A32, perm, nrm32, (float *)nrmd);
@@ -3662,13 +3930,9 @@ __global__ void __launch_bounds__(1024) k_svd(int m, int k, const double2 *__res
         X[e] = i >= j ? make_float2(r.x, -r.y) : make_float2(0.f, 0.f);
     }
     __syncthreads();
-    // the columns in registers where a warp has a pair of its own and two rows a lane hold them (the
-    // exchange buffers take Ad's place, free until phase 2)
     int s32;
-    if (m <= 64 && m >= 16 && (m + 1) / 2 <= (nt >> 5))
-        s32 = jacobi_regs_f32(m, X, (float2 *)Ad, reg_nx, tol32, 40, &s_flag, &s_off);
-    else
-        s32 = jacobi_sweeps_f32(m, m, X, nullptr, nrm32, tol32, 40, &s_flag, &s_off, tab32);
+    if constexpr (clustered) s32 = jacobi_cluster_f32(m, X, (float2 *)ex, tol32, 40, &s_fl);
+    else s32 = jacobi_sweeps_f32(m, m, X, nullptr, nrm32, tol32, 40, &s_flag, &s_off, tab32);
     {
         const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
         for (int c = warp; c < m; c += nwarps) {
@@ -3830,8 +4094,11 @@ __global__ void __launch_bounds__(1024) k_svd(int m, int k, const double2 *__res
     // Two sweeps when the FP32 vectors are good (the 64 x 64 Helmholtz Hessenbergs); where FP32
     // could not resolve the small singular values (condition ~1e6 and up) it takes more: 11 for
     // m = 96 over six decades.
-    const int sdf = jacobi_polish_df(m, Ad, Vd, ldv, nrmd, 4.0f * 2.220446e-16f * m, 30, &s_flag, &s_off, ptab, pcnt,
-                                     flag_list, k, coefs);
+    int sdf;
+    if constexpr (clustered)
+        sdf = jacobi_polish_cluster(m, Ad, Vd, ldv, nrmd, toldf, 30, small_col, flag_list, k, coefs, ex, &s_fl);
+    else
+        sdf = jacobi_polish_df(m, Ad, Vd, ldv, nrmd, toldf, 30, &s_flag, &s_off, ptab, pcnt, flag_list, k, coefs);
     // singular values in descending order (ties broken by column index); the output vectors are
     // the flagged columns, the only ones polished, in descending order of their values
     // (NaN values sort as -inf: ranks and slots stay permutations, every slot is written)
@@ -5511,10 +5778,31 @@ void launch_svd_smallest(int m, int k, const double2 *H, size_t strideH, const i
     Launch L_(KC_SVD, (double)sizeof(double2) * (m + 1.0) * m, st, 1);
     size_t smem = svd_smem_bytes(m);
     int use_smem = smem <= 200 * 1024;
-    if (use_smem) allow_smem(k_svd, smem);
+    if (use_smem) allow_smem(k_svd<false>, smem);
     const int pairs = (m + 1) / 2;
-    int threads = 32 * (pairs < 32 ? (pairs > 4 ? pairs : 4) : 32);
-    k_svd<<<1, threads, use_smem ? smem : 0, st>>>(m, k, H, strideH, lead, vs, sigma, work, use_smem, sweeps);
+    const int threads = 32 * (pairs < 32 ? (pairs > 4 ? pairs : 4) : 32);
+    // 40 to 63 columns: a cluster of 4 CTAs up to 24 pairs, 8 above, where the exchange buffers fit beside the
+    // work.  In clocks, one CTA against the cluster: m = 30, k = 8: 578 to 650 thousand; m = 40, k = 10: 1070 to
+    // 1028; m = 48, k = 24: 1717 to 1355; m = 60, k = 20: 2430 to 1755 (below, a round is one pair's latency)
+    const int nc = m < 40 || m > 63 ? 1 : pairs <= 24 ? 4 : 8, wpc = (pairs + nc - 1) / nc;
+    const size_t exch = sizeof(dfc) * 4 * (size_t)wpc * (2 * m + 2);
+    if (nc > 1 && smem + exch <= 220 * 1024) {
+        allow_smem(k_svd<true>, smem + exch);
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(nc);
+        cfg.blockDim = dim3(SVD_CLUSTER_THREADS);
+        cfg.dynamicSmemBytes = smem + exch;
+        cfg.stream = st;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = nc;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        cudaLaunchKernelEx(&cfg, k_svd<true>, m, k, H, strideH, lead, vs, sigma, work, 1, sweeps);
+        return;
+    }
+    k_svd<false><<<1, threads, use_smem ? smem : 0, st>>>(m, k, H, strideH, lead, vs, sigma, work, use_smem, sweeps);
 }
 
 // Algorithmic bytes of the fused Krylov loop: per step the operator product, the projection
