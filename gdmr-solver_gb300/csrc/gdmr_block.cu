@@ -121,7 +121,8 @@ __device__ __forceinline__ float scatter12(float (&v)[12], int lane) {
 
 // part[slot][G][6 i + 2 b + (re | im)]: <v_i, y_b> for the nv basis vectors, then <y_a, y_b>; y_b is
 // basis slot nv + b.  HBM-bound: a CTA keeps the block's elements of a chunk in registers and streams
-// the basis past them two vectors at a time.  FP32 sums over 256 elements a warp, then double-float.
+// the basis past them two vectors at a time: 96^3, 64 systems, nv = 13: 1083 us with the finish, 6.69 TB/s of its
+// bytes (1185 us with four elements a thread).  FP32 sums over 256 elements a warp, then double-float.
 template <int EPT, int VEC>
 __global__ void __launch_bounds__(NTB, 2)
     k_block_proj(int n, int nv, const float2 *__restrict__ V0, size_t strideV, const int *__restrict__ act,
@@ -197,12 +198,13 @@ __global__ void __launch_bounds__(NTB, 2)
 }
 
 // v_new_b = sum_a y_a T_ab - sum_i v_i D_ib in place of y_b (basis slots nv .. nv + 2).  HBM-bound:
-// reads nv + 3 vectors, writes three.  A zero T_bb (a system that broke down earlier) stores zeros.
+// reads nv + 3 vectors, writes three.  96^3, 64 systems, nv = 13: 1220 us, 7.06 TB/s of its bytes (1258 us with two
+// vectors in flight; four elements a thread instead of eight: 1225-1390).  A zero T_bb (a system that broke down earlier) stores zeros.
 template <int EPT, int VEC>
 __global__ void __launch_bounds__(NTB, 2)
     k_block_update(int n, int nv, float2 *__restrict__ V0, size_t strideV, const int *__restrict__ act,
                    const float2 *__restrict__ dco, size_t dstride) {
-    constexpr int NP = EPT / VEC, PU = 2;
+    constexpr int NP = EPT / VEC, PU = 4;
     __shared__ float2 ds[BK_S * BK_QMAX], ts[BK_S * BK_S];
     const int slot = blockIdx.x, s = act[slot], tid = threadIdx.x;
     float2 *V = V0 + (size_t)s * strideV;
@@ -263,9 +265,6 @@ __global__ void __launch_bounds__(NTB, 2)
     }
 }
 
-__device__ __forceinline__ double2 zmul(double2 a, double2 b) {
-    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
 __device__ __forceinline__ double2 zfma(double2 a, double2 b, double2 c) {
     return make_double2(::fma(a.x, b.x, ::fma(-a.y, b.y, c.x)), ::fma(a.x, b.y, ::fma(a.y, b.x, c.y)));
 }
@@ -277,7 +276,7 @@ __device__ __forceinline__ double wsum(double v) {
 
 // One CTA a system: the block's coefficients from the partial sums, the Cholesky factor, the
 // update's coefficients (dco: T then D) and the block's Hessenberg columns.  Latency-bound.
-constexpr int NTF = 512;
+template <int NTF>
 __global__ void __launch_bounds__(NTF) k_block_finish(int nv, int kk, int m, int G, const double *__restrict__ part,
                                                       const int *__restrict__ act, SysState *state,
                                                       double2 *__restrict__ H0, size_t strideH,
@@ -514,8 +513,10 @@ void launch_block_step(int n, int nv, int kk, int m, float2 *V, size_t strideV, 
     const int sms = device_sm_count(), ept = block_ept(n, nsys, sms);
     const int nch = (n + NTB * ept - 1) / (NTB * ept);
     const bool v2 = n % 2 == 0 && strideV % 2 == 0 && (reinterpret_cast<uintptr_t>(V) & 15) == 0;
-    // about eight CTAs an SM over the launch: a CTA's chunks share one set of partial sums
-    const int G = (int)std::min<long>(nch, std::max<long>(1, ((long)sms * 8 + nsys - 1) / nsys));
+    // about eight CTAs an SM over the launch, two a system and SM at most: a CTA's chunks share one set of
+    // partial sums, and one CTA adds a system's (one system at 128^3, nv = 21: 150 us with 1024 sets; 64 systems
+    // at 96^3 1335 us with half as many, 1083 as is)
+    const int G = (int)std::min<long>(nch, std::min<long>(2 * sms, ((long)sms * 8 + nsys - 1) / nsys));
     const size_t smem = sizeof(dfr) * NWB * BK_C * (size_t)(nv + BK_S);
     float2 *dco = reinterpret_cast<float2 *>(scratch + capacity - krylov_block_scratch(m, nsys));
     const size_t dstride = BK_S * BK_S + (size_t)BK_S * (m + 1);
@@ -527,8 +528,14 @@ void launch_block_step(int n, int nv, int kk, int m, float2 *V, size_t strideV, 
         };
         if (ept == EPT_BIG) v2 ? go(k_block_proj<EPT_BIG, 2>) : go(k_block_proj<EPT_BIG, 1>);
         else v2 ? go(k_block_proj<EPT_SMALL, 2>) : go(k_block_proj<EPT_SMALL, 1>);
-        k_block_finish<<<nsys, NTF, 0, st>>>(nv, kk, m, G, scratch, act, state, H, strideH, a[0], a[1], a[2], strideC, tol,
-                                             dco, dstride);
+        // more threads only where there are many sets to add (12 systems, 49 sets: 57 us with the projection at 512
+        // threads, 61 at 1024)
+        auto fin = [&](auto kernel, int threads) {
+            kernel<<<nsys, threads, 0, st>>>(nv, kk, m, G, scratch, act, state, H, strideH, a[0], a[1], a[2], strideC,
+                                             tol, dco, dstride);
+        };
+        if (G > 128) fin(k_block_finish<1024>, 1024);
+        else fin(k_block_finish<512>, 512);
     }
     ProfScope p(KC_UPDATE, sizeof(float2) * (double)n * nsys * (nv + 2 * BK_S), st, 1);
     const dim3 grid(nsys, nch);
