@@ -3247,8 +3247,10 @@ __device__ __forceinline__ void max_remote(unsigned a, int v) {
 // are dealt to the cluster's CTAs, wpc warps each, every warp keeping its two columns in registers, two rows a
 // lane (at most 64 rows).  A round ends by handing the columns on along the circle (the top row to the right,
 // the bottom row to the left) through the receiving CTA's shared memory, double-buffered, with one cluster
-// barrier.  Slot w of the circle (the pair of warp w of the cluster) starts with columns w and mm - 1 - w, and
-// after a sweep's mm - 1 rounds every column is back.
+// barrier.  Slot w of the circle (the pair of warp w of the cluster) starts with the columns that give every round
+// the pairs of pair_table, and after a sweep's mm - 1 rounds every column is back.  (With the table's rounds in
+// reverse, which the two rows one way round give, the pivoted columns take a sweep more, 8 instead of 7 at m = 48,
+// k = 24, and vectors of a small k come out ten times further off at m = 55, k = 8.)
 struct CircleSlot {
     int np, wpc, w;          // pairs, pairs a CTA, this warp's pair
     unsigned rank;
@@ -3293,7 +3295,7 @@ __device__ int jacobi_cluster_f32(int m, float2 *X, float2 *ex, float tol, int m
     const unsigned half = (unsigned)(2 * cs.wpc * stride * sizeof(float2));
     const float2 *my = ex + warp * stride;
     cluster_barrier();                                        // CTA 0's X is complete
-    int ip = cs.w, iq = mm - 1 - cs.w;
+    int ip = cs.w ? mm - 1 - cs.w : 0, iq = cs.w ? cs.w : mm - 1;
     float2 p0 = make_float2(0.f, 0.f), p1 = p0, q0 = p0, q1 = p0;
     if (cs.mine) {
         if (r0) ld_remote(x0 + (ip * m + lane) * 8, p0);
@@ -3713,7 +3715,7 @@ __device__ int jacobi_polish_cluster(int m, dfc *A, dfc *V, int ldv, dfr *nrm, f
         hi = __ballot_sync(0xffffffffu, b1 != 0);
     }
     auto flagged = [&](int c) { return ((c < 32 ? lo >> c : hi >> (c - 32)) & 1u) != 0; };
-    int ip = cs.w, iq = mm - 1 - cs.w;
+    int ip = cs.w ? mm - 1 - cs.w : 0, iq = cs.w ? cs.w : mm - 1;
     dfc pa[2] = {z, z}, pv[2] = {z, z}, qa[2] = {z, z}, qv[2] = {z, z};
     if (cs.mine) {
         if (a0) ld_remote(A0 + (ip * rows + lane) * 16, pa[0]);
@@ -3764,18 +3766,16 @@ __device__ int jacobi_polish_cluster(int m, dfc *A, dfc *V, int ldv, dfr *nrm, f
                 if (max(ip, iq) < m && (flagged(ip) || flagged(iq))) {
                     dfr gr(0.f, 0.f), gi(0.f, 0.f);
 #pragma unroll
-                    for (int u = 0; u < 2; ++u) {             // unnormalised chains, canonical below
-                        gr = rfma(pa[u].x, qa[u].x, gr);
-                        gr = rfma(pa[u].y, qa[u].y, gr);
-                        gi = rfma(pa[u].x, qa[u].y, gi);
-                        gi = rfma(-pa[u].y, qa[u].x, gi);
+                    for (int u = 0; u < 2; ++u) {
+                        gr = fma(pa[u].x, qa[u].x, gr);
+                        gr = fma(pa[u].y, qa[u].y, gr);
+                        gi = fma(pa[u].x, qa[u].y, gi);
+                        gi = fma(-pa[u].y, qa[u].x, gi);
                     }
                     // the two sums share one butterfly (lower half re, upper half im); the two-sum is
                     // symmetric, so every lane ends with the same values
                     {
                         const bool up = lane & 16;
-                        gr = df_renorm(gr.hi, gr.lo);
-                        gi = df_renorm(gi.hi, gi.lo);
                         const dfr give = up ? gr : gi;
                         dfr v = (up ? gi : gr) + dfr(__shfl_xor_sync(0xffffffffu, give.hi, 16),
                                                      __shfl_xor_sync(0xffffffffu, give.lo, 16));
@@ -4039,16 +4039,16 @@ __global__ void __launch_bounds__(clustered ? SVD_CLUSTER_THREADS : 1024) k_svd(
     dfc *T = Sc;                            // m x m, leading dimension m
     for (int e = tid; e < m * m; e += nt) {
         const int i = e % m, j = e / m;     // T[i][j] = sum_l V[i][l] F[l][j]
-        dfr sx(0.f, 0.f), sy(0.f, 0.f);     // unnormalised chains, canonical at the end
+        dfr sx(0.f, 0.f), sy(0.f, 0.f);
         for (int l = 0; l < m; ++l) {
             const dfc v = Vd[(size_t)l * ldv + i], f = E[(size_t)j * m + l];
-            sx = rfma(dfr(v.x.hi, 0.f), f.x, sx);
-            sx = rfma(dfr(-v.y.hi, 0.f), f.y, sx);
-            sy = rfma(dfr(v.x.hi, 0.f), f.y, sy);
-            sy = rfma(dfr(v.y.hi, 0.f), f.x, sy);
+            sx = fma(dfr(v.x.hi, 0.f), f.x, sx);
+            sx = fma(dfr(-v.y.hi, 0.f), f.y, sx);
+            sy = fma(dfr(v.x.hi, 0.f), f.y, sy);
+            sy = fma(dfr(v.y.hi, 0.f), f.x, sy);
         }
-        T[e].x = df_renorm(sx.hi, sx.lo);
-        T[e].y = df_renorm(sy.hi, sy.lo);
+        T[e].x = sx;
+        T[e].y = sy;
     }
     __syncthreads();
     for (int e = tid; e < m * m; e += nt) {
@@ -4061,20 +4061,19 @@ __global__ void __launch_bounds__(clustered ? SVD_CLUSTER_THREADS : 1024) k_svd(
     for (int i = tid; i < rows * m; i += nt) Hd[i] = to_dfc(make_double2(H[i].x * sc, H[i].y * sc));
     __syncthreads();
     for (int e = tid; e < rows * m; e += nt) {
-        // A[r][c] = sum_p H[r][p] V[p][c]; unnormalised chains, canonical at the end
+        // A[r][c] = sum_p H[r][p] V[p][c]; normalised chains: every error of the small singular values
+        // and their vectors starts here (unnormalised ones left values off by 2e-15 ||H|| instead of 5e-16)
         const int r = e % rows, c = e / rows;
         dfr sx(0.f, 0.f), sy(0.f, 0.f);
         for (int p = 0; p < m; ++p) {
             const dfc h = Hd[(size_t)p * rows + r], v = Vd[(size_t)c * ldv + p];
-            sx = rfma(h.x, v.x, sx);
-            sx = rfma(-h.y, v.y, sx);
-            sy = rfma(h.x, v.y, sy);
-            sy = rfma(h.y, v.x, sy);
+            sx = fma(h.x, v.x, sx);
+            sx = fma(-h.y, v.y, sx);
+            sy = fma(h.x, v.y, sy);
+            sy = fma(h.y, v.x, sy);
         }
-        dfc a;
-        a.x = df_renorm(sx.hi, sx.lo);
-        a.y = df_renorm(sy.hi, sy.lo);
-        Ad[e] = a;
+        Ad[e].x = sx;
+        Ad[e].y = sy;
     }
     __syncthreads();
     // 3. double-float polish of the k smallest.  Sc (H no longer needed) takes the packed pair
