@@ -233,6 +233,11 @@ int sell_from_csr(DeviceSell &out, int n, const int *rowptr, const int *colidx, 
             vdf[e].y = dfr(im);
         }
     };
+    // pattern index of an offset; rows mostly hold the pattern in order, so the one after the last comes first
+    auto entry = [&](int off, int guess) {
+        if (guess < np && pat[guess] == off) return guess;
+        return (int)(std::find(pat.begin(), pat.end(), off) - pat.begin());
+    };
     for (int s = 0; s < ns; ++s) {
         const int w = (sp[s + 1] - sp[s]) / 32;
         for (int lane = 0; lane < 32; ++lane) {
@@ -241,9 +246,9 @@ int sell_from_csr(DeviceSell &out, int n, const int *rowptr, const int *colidx, 
             for (int q = beg; q < beg + len; ++q) band = std::max(band, std::abs(colidx[q] - r));
             if (uni[s]) {
                 // pattern order; duplicate entries of one column add up, as in CSR
-                std::vector<double> re(np, 0.0), im(np, 0.0);
-                for (int q = beg; q < beg + len; ++q) {
-                    const int e = (int)(std::find(pat.begin(), pat.end(), colidx[q] - r) - pat.begin());
+                double re[SELL_PATTERN] = {}, im[SELL_PATTERN] = {};
+                for (int q = beg, e = -1; q < beg + len; ++q) {
+                    e = entry(colidx[q] - r, e + 1);
                     re[e] += vals_ri[2 * (size_t)q];
                     im[e] += vals_ri[2 * (size_t)q + 1];
                 }
@@ -272,8 +277,9 @@ int sell_from_csr(DeviceSell &out, int n, const int *rowptr, const int *colidx, 
     bool same = gx > 0;
     if (gx)
         for (int r = 0; r < n; ++r)
-            for (int q = rowptr[r]; q < rowptr[r + 1]; ++q) {
-                const size_t e = (size_t)(std::find(pat.begin(), pat.end(), colidx[q] - r) - pat.begin());
+            for (int q = rowptr[r], e0 = -1; q < rowptr[r + 1]; ++q) {
+                e0 = entry(colidx[q] - r, e0 + 1);
+                const size_t e = (size_t)e0;
                 const double re = vals_ri[2 * (size_t)q], im = vals_ri[2 * (size_t)q + 1];
                 double &a = gre[e * n + r], &b = gim[e * n + r];
                 Plane &f = first[e];
