@@ -585,7 +585,7 @@ def main():
     op_kernel = ("matrix-free stencil (k_stencil)" if args.stencil else
                  f"structured grid (k_grid_spmm, {args.grid_batch} systems a thread)"
                  if sysm.grid_shape() and not args.sell and args.grid_batch else
-                 "SELL-32 (k_spmm) for the batch, structured grid (k_grid_spmm) for single vectors"
+                 "structured grid with constant planes (k_grid_const)"
                  if sysm.grid_shape() and not args.sell else "SELL-32 (k_spmm, k_spmv2)")
     Bd = torch.from_numpy(B).to(f"cuda:{local}")
     Xd = torch.zeros_like(Bd)
