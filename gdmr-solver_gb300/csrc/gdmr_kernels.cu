@@ -5652,12 +5652,16 @@ void launch_wdeflate(int n, int kk, const float2 *W, const float2 *y, size_t str
     // 0: the tensor cores; 1-3: the update kernels (grouped over 4 or 2 systems, one system a CTA)
     const bool tc = wapply_tc_ok(n, kk, nsys);
     static const int update_variant[4] = {1, 6, 7, 1};
+    // the third product of a block may leave the FP32 range where the Krylov space is exhausted, which
+    // k_block_finish finds and drops; a norm of it must not mark the system non-finite
+    FinishArgs f{};
+    f.mode = FIN_DISCARD;
     auto run = [&](int v) {
         if (v == 0 && tc)
             launch_wapply_sub_tc(n, kk, W, coef, strideC, act, nsys, y, strideY, out, strideO, st);
         else
             update_dispatch<float>(update_variant[v], n, W, kk, nullptr, 0, 0, y, strideY, out, strideO, act, nsys,
-                                   coef, strideC, partials, tickets, state, FinishArgs{}, false, st);
+                                   coef, strideC, partials, tickets, state, f, false, st);
     };
     int v = 0;
     if (nsys > 1 && !profile_enabled()) v = tuned_variant(prec_key<float>(), 2, n, nsys, kk, 0, 4, st, run);

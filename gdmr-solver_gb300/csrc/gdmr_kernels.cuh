@@ -107,6 +107,7 @@ enum FinishMode : int {
     FIN_DEFLATION = 2,  // deflation step: H[i,i] = <w,Az>/||w||, alpha
     FIN_UNIT = 3,       // alpha = 1/||w||
     FIN_RESIDUAL = 4,   // cycle end: rho, alpha = 1/rho
+    FIN_DISCARD = 5,    // the state is left alone (the deflator: its vectors need no norm)
 };
 
 struct FinishArgs {
@@ -129,6 +130,7 @@ struct FinishArgs {
 // then, per mode, the Hessenberg column with the breakdown test and the reference's identity
 // tail (gDMR.cu:2256-2289), the deflation loop's diagonal, or the cycle-end residual factor.
 __device__ inline void run_finish(const FinishArgs &f, int s, SysState &st, double n2, double cre, double cim) {
+    if (f.mode == FIN_DISCARD) return;
     st.nrm2 = n2;
     st.cross_re = cre;
     st.cross_im = cim;
