@@ -1106,6 +1106,8 @@ int Engine<R>::refine_admit(int slot, const double2 *b, const double2 *x0, doubl
     if (x0) GDMR_CK(cudaMemcpyAsync(slot_x(slot), x0, vb, cudaMemcpyDeviceToDevice, stream));
     else GDMR_CK(cudaMemsetAsync(slot_x(slot), 0, vb, stream));
     GDMR_CK(cudaMemsetAsync(X_ + (size_t)slot * n_, 0, sizeof(C) * (size_t)n_, stream));
+    // the non-finite mark is the last right-hand side's
+    GDMR_CK(cudaMemsetAsync(&state_[slot].bad, 0, sizeof(int), stream));
     Slot &S = slot_[slot];
     S = Slot();
     S.active = true;
