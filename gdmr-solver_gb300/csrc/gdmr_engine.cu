@@ -1080,7 +1080,7 @@ template <class R> int Engine<R>::refine_setup(const SellMatrix &A64) {
         return GDMR_EINVAL;
     }
     A64_ = A64;
-    front_done_ = false;
+    if (discard_front(true) != GDMR_OK) return GDMR_ECUDA;
     if (!r64_) {
         int rc;
         if ((rc = alloc((void **)&r64_, sizeof(double2) * (size_t)n_ * cap_)) != GDMR_OK) return rc;
@@ -1093,6 +1093,14 @@ template <class R> int Engine<R>::refine_setup(const SellMatrix &A64) {
     blocks_on_ = cholqr_on_ = true;
     GDMR_CK(cudaMemsetAsync(X_, 0, sizeof(C) * (size_t)n_ * cap_, stream));
     return begin_solve();
+}
+
+// A deflation loop enqueued ahead of a cycle that will not use it: its failed factor, if it has one, is no
+// later cycle's.
+template <class R> int Engine<R>::discard_front(bool always) {
+    if (front_done_ || always) GDMR_CK(cudaMemsetAsync(&state_[cap_].ill, 0, sizeof(int), stream));
+    front_done_ = false;
+    return GDMR_OK;
 }
 
 template <class R>
@@ -1217,7 +1225,7 @@ template <class R> int Engine<R>::refine_cycle(std::vector<int> *done) {
     }
     act_h_ = next;
     if (next.empty()) {
-        front_done_ = false;
+        if (discard_front(false) != GDMR_OK) return GDMR_ECUDA;
         return sync_deflation();
     }
     if (set_active(next) != GDMR_OK) return GDMR_ECUDA;
@@ -1229,7 +1237,8 @@ template <class R> int Engine<R>::refine_cycle(std::vector<int> *done) {
     launch_demote_unit<R>(n, r64_, n, R_, n, V_, strideV(), act_, na, state_, stream);
     k_cycle_reset<<<1, 256, 0, stream>>>(act_, na, state_, 1);
     const int kk = (k > 0 && have_z_) ? k : 0;
-    if (kk == 0) front_done_ = false;   // the deflation space was dropped after a timeout
+    // the deflation space was dropped after a timeout
+    if (kk == 0 && discard_front(false) != GDMR_OK) return GDMR_ECUDA;
     g_direct_ = !restart_vectors(next, kk);
     long mv = 0;
     // breakdown of unit vectors: an invariant subspace at working precision
@@ -1408,7 +1417,7 @@ template <class R> int Engine<R>::multi_back(cudaEvent_t after) {
     GDMR_CK(cudaStreamWaitEvent(stream, after, 0));
     int rc = enqueue_back(mf_kk_, mf_nsys_, false);
     if (rc != GDMR_OK) return rc;
-    launch_refine_update<R>(n_, x64_, n_, X_, n_, act_, mf_nsys_, state_, cap_, stream);
+    launch_refine_update<R>(n_, x64_, n_, X_, n_, act_, mf_nsys_, state_, -1, stream);
     GDMR_CK(cudaGetLastError());
     mf_ran_ = true;
     return GDMR_OK;

@@ -254,6 +254,7 @@ template <class R> class Engine {
     cudaEvent_t ev_x_ = nullptr, ev_res_ = nullptr;
     double2 *partials_res_ = nullptr;
     bool front_done_ = false;
+    int discard_front(bool always);
     void enqueue_deflation_loop(int kk, long *matvecs);
     bool graph_ok(int nsys) const;
     // restart-cycle graphs (key: deflation dimension, batch size, Z buffer parity, tolerance)

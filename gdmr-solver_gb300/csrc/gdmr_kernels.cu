@@ -4612,7 +4612,7 @@ __global__ void __launch_bounds__(NT) k_refine_update(int n, double2 *__restrict
     using C = typename CT<R>::t;
     const int s = act[blockIdx.y];
     const double sc = state[s].true_res;
-    const bool drop = state[s].ill != 0 || state[shared].ill != 0;   // the cycle's correction is not used
+    const bool drop = state[s].ill != 0 || (shared >= 0 && state[shared].ill != 0);   // the cycle's correction is not used
     double2 *x = x0 + (size_t)s * strideX;
     C *d = d0 + (size_t)s * strideD;
     for (long i = (long)blockIdx.x * NT + threadIdx.x; i < n; i += (long)gridDim.x * NT) {

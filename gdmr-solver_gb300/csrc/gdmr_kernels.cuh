@@ -558,7 +558,7 @@ template <class R>
 void launch_copy_vec(int n, const typename CT<R>::t *src, size_t strideS, typename CT<R>::t *dst, size_t strideD,
                      const int *act, int nsys, cudaStream_t st);
 // x64_s += scale_s * d_s (d complex64/128 inner correction), then d_s = 0; no correction where the system
-// or the shared pseudo-system state[shared] is flagged ill.
+// or the shared pseudo-system state[shared] (none if shared < 0) is flagged ill.
 template <class R>
 void launch_refine_update(int n, double2 *x, size_t strideX, typename CT<R>::t *d, size_t strideD,
                           const int *act, int nsys, const SysState *state, int shared, cudaStream_t st);

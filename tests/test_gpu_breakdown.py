@@ -51,3 +51,42 @@ def test_space_exhausted_at_the_last_single_step(nrhs):
     X, stats = s.solve_batch(B, tol=TOL, max_cycles=200)
     _check(A, B, X, stats)
     s.close()
+
+
+@pytest.mark.parametrize("after", ["solve", "multi"])
+def test_factor_that_failed_in_an_unused_loop_is_forgotten(after):
+    # with the overlapped residual, the deflation loop of a next cycle is enqueued before the host knows
+    # that every system is done (zero right-hand sides are, at once); its factor fails on a singular space
+    A = problems.helmholtz((20, 19, 18), 5.0, 0.1)
+    B = _rhs(A.n, 2)
+    Z = _rhs(A.n, 16, 900)
+    Z[9] = Z[3]
+
+    def system():
+        s = gdmr.System(A, 40, 16, capacity=2, precision="mixed")
+        s.set_graphs(False)
+        return s
+
+    s = system()
+    ref = [t["cycles"] for t in s.solve_batch(B, tol=TOL, max_cycles=200)[1]]
+    s.close()
+    s = system()
+    s.solve_batch(B, tol=TOL, max_cycles=200)
+    s.import_deflation(Z)
+    prev = gdmr.overlap_residual(1)
+    try:
+        assert [t["cycles"] for t in s.solve_batch(np.zeros_like(B), tol=TOL, max_cycles=200)[1]] == [0, 0]
+    finally:
+        gdmr.overlap_residual(prev)
+    s.drop_deflation()
+    if after == "solve":
+        stats = s.solve_batch(B, tol=TOL, max_cycles=200)[1]
+        assert [t["cycles"] for t in stats] == ref
+    else:
+        prev = gdmr.multi_tail(0)      # lockstep to the end
+        try:
+            (X, stats), = gdmr.multi_solve([s], [B], tol=TOL, max_cycles=200)
+        finally:
+            gdmr.multi_tail(prev)
+    assert [t["status"] for t in stats] == [0, 0], stats
+    s.close()
