@@ -403,6 +403,9 @@ extern "C" int gdmrLastHistory(gdmr_cycle *out, int max) {
 }
 
 extern "C" long long gdmrKernelLaunches(void) { return launch_count(); }
+extern "C" void gdmrCycleCounts(long long *counts) {
+    for (int i = 0; i < CC_NUM; ++i) counts[i] = cycle_count(i);
+}
 extern "C" unsigned gdmrAsyncTimeouts(void) { return wproj_tc_timeouts() + bulk_timeouts(); }
 extern "C" double gdmrWaitLimit(double ms) {
     const double prev = wait_limit_ms();

@@ -38,6 +38,8 @@ const char *last_error() {
 namespace {
 std::atomic<int> g_alloc_countdown{0};   // > 0: the allocation that takes it to 0 fails
 }
+static std::atomic<long long> g_cycle_counts[CC_NUM];
+long long cycle_count(int which) { return g_cycle_counts[which].load(); }
 void inject_alloc_failure(int nth) { g_alloc_countdown.store(nth > 0 ? nth : 0); }
 
 // NVTX ranges around the phases of a solve (free when no tool is attached).
@@ -643,10 +645,11 @@ template <class R> int Engine<R>::run_cycle(int kk, int nsys, int lead, double t
     ++cycles_run_;
     if (!graphable) return enqueue_cycle(kk, nsys, tol, matvecs, false);
     const int zpar = zpar_;
+    const bool blocked = blocked_ok(kk, nsys), cholqr = cholqr_ok(kk);
     cudaGraphExec_t exec = nullptr;
     for (auto &g : graphs_)
-        if (g.kk == kk && g.nsys == nsys && g.zpar == zpar && g.tol == tol && g.blocked == blocked_ &&
-            g.cholqr == cholqr_on_ && g.gdirect == g_direct_)
+        if (g.kk == kk && g.nsys == nsys && g.zpar == zpar && g.tol == tol && g.blocked == blocked &&
+            g.cholqr == cholqr && g.gdirect == g_direct_)
             exec = g.exec;
     if (!exec) {
         if (graphs_.size() >= 32) {
@@ -674,7 +677,7 @@ template <class R> int Engine<R>::run_cycle(int kk, int nsys, int lead, double t
             set_last_error(GDMR_ECUDA, std::string("restart-cycle graph: ") + cudaGetErrorString(e));
             return GDMR_ECUDA;
         }
-        graphs_.push_back(GraphEntry{kk, nsys, zpar, tol, blocked_, cholqr_on_, g_direct_, exec});
+        graphs_.push_back(GraphEntry{kk, nsys, zpar, tol, blocked, cholqr, g_direct_, exec});
     }
     GDMR_CK(cudaGraphLaunch(exec, stream));
     // the graph joins the deflation update into the main stream: the new Z is ready in order
@@ -743,11 +746,9 @@ template <class R> void Engine<R>::enqueue_deflation_loop(int kk, long *matvecs)
     // batched product straight into W's slots (the matrix read once, not kk times); step i
     // then orthogonalises slot i against the finished slots 0..i-1 and normalises it in place
     const bool batched = op.kind == Operator<R>::SELL || op.kind == Operator<R>::STENCIL;
-    if constexpr (std::is_same<R, float>::value) {
-        if (batched && cholqr_ok(kk)) {
-            enqueue_deflation_cholqr(kk, matvecs);
-            return;
-        }
+    if (cholqr_ok(kk)) {
+        enqueue_deflation_cholqr(kk, matvecs);
+        return;
     }
     if (batched) {
         *matvecs += kk;
@@ -780,7 +781,9 @@ template <class R> void Engine<R>::enqueue_deflation_loop(int kk, long *matvecs)
 // 0.45 ms of a 3.1 ms cycle for 16 vectors of 100,345, against 0.1 ms; 0.8 against 0.5 ms for 24 of
 // 884,736.  Z holds approximate singular vectors, so the columns of A Z are nearly orthogonal.
 template <class R> bool Engine<R>::cholqr_ok(int kk) const {
+    if constexpr (!std::is_same<R, float>::value) return false;
     return refined_ && cholqr_on_ && kk <= CHOLQR_MAX && wapply_tc_ok(n_, kk, kk) &&
+           (op.kind == Operator<R>::SELL || op.kind == Operator<R>::STENCIL) &&
            (size_t)kk * kk * 2 * (((size_t)n_ + 2047) / 2048) <= scratch_size(partials_);
 }
 template <class R> void Engine<R>::enqueue_deflation_cholqr(int kk, long *matvecs) {
@@ -1090,7 +1093,7 @@ template <class R> int Engine<R>::refine_setup(const SellMatrix &A64) {
     slot_.assign(cap_, Slot());
     act_h_.clear();
     kk_prev_ = 0;
-    blocks_on_ = cholqr_on_ = true;
+    cholqr_on_ = true;
     GDMR_CK(cudaMemsetAsync(X_, 0, sizeof(C) * (size_t)n_ * cap_, stream));
     return begin_solve();
 }
@@ -1243,7 +1246,10 @@ template <class R> int Engine<R>::refine_cycle(std::vector<int> *done) {
     long mv = 0;
     // breakdown of unit vectors: an invariant subspace at working precision
     const double inner_tol = sizeof(R) == 4 ? 1e-6 : 1e-14;
-    blocked_ = blocks_on_;
+    blocked_ = true;
+    for (int s : next) blocked_ = blocked_ && !slot_[s].stepwise;
+    if (blocked_ok(kk, na)) g_cycle_counts[CC_BLOCKED] += na;
+    if (cholqr_ok(kk)) ++g_cycle_counts[CC_FACTORED];
     const bool had_z = have_z_;
     const int cycle_rc = run_cycle(kk, na, lead, inner_tol, &mv);
     blocked_ = g_direct_ = false;
@@ -1252,6 +1258,7 @@ template <class R> int Engine<R>::refine_cycle(std::vector<int> *done) {
     if (read_state(cap_ + 1) != GDMR_OK) return GDMR_ECUDA;
     const bool factor_failed = hstate_[cap_].ill != 0;   // the deflation loop's: no system has a cycle
     if (factor_failed) {
+        ++g_cycle_counts[CC_FACTOR_FAILED];
         cholqr_on_ = false;
         GDMR_CK(cudaMemsetAsync(&state_[cap_].ill, 0, sizeof(int), stream));
     }
@@ -1269,8 +1276,11 @@ template <class R> int Engine<R>::refine_cycle(std::vector<int> *done) {
         Slot &S = slot_[s];
         const SysState &st = hstate_[s];
         if (factor_failed || st.ill) {
-            // no correction; the blocked steps, if they gave up on this system, step by step from now on
-            if (!factor_failed) blocks_on_ = false;
+            // no correction; the blocked steps, if they gave up on this system, step by step while it is in flight
+            if (!factor_failed) {
+                ++g_cycle_counts[CC_DROPPED];
+                S.stepwise = true;
+            }
             S.loop_flag = 0;
             S.stats.cycles += 1;
             S.stats.matvecs += m;

@@ -101,6 +101,10 @@ struct CycleRecord {
     int stagnated = 0;    // 1: rho > 0.995, the reference's stagnation flag (gDMR.cu:2506)
 };
 
+// Process-wide counts of the refined cycles' fast forms (gdmrCycleCounts).
+enum CycleCount { CC_BLOCKED = 0, CC_DROPPED = 1, CC_FACTORED = 2, CC_FACTOR_FAILED = 3, CC_NUM = 4 };
+long long cycle_count(int which);
+
 struct SolveStats {
     int cycles = 0;
     int its = 0;             // reference convention: cycles - 1
@@ -229,6 +233,7 @@ template <class R> class Engine {
     // refined form
     struct Slot {
         bool active = false;
+        bool stepwise = false;   // a block was ill-conditioned: step by step until this right-hand side leaves
         int loop_flag = 0, flag_count = 0, max_cycles = 0;
         double bnorm = 0, tol = 0;
         SolveStats stats;
@@ -257,7 +262,8 @@ template <class R> class Engine {
     int discard_front(bool always);
     void enqueue_deflation_loop(int kk, long *matvecs);
     bool graph_ok(int nsys) const;
-    // restart-cycle graphs (key: deflation dimension, batch size, Z buffer parity, tolerance)
+    // restart-cycle graphs (key: deflation dimension, batch size, Z buffer parity, tolerance, and the forms of
+    // the Krylov and deflation loops and of the residual's coordinates)
     struct GraphEntry {
         int kk, nsys, zpar;
         double tol;
@@ -271,16 +277,15 @@ template <class R> class Engine {
     int enqueue_front(int kk, int nsys, long *matvecs);
     int enqueue_krylov(int kk, int nsys, double tol, long *matvecs);
     int enqueue_back(int kk, int nsys, bool join);
-    // Blocked Krylov steps: blocked_ is set around a refined complex64 cycle while blocks_on_ (from
-    // refine_setup until a system's block turns out ill-conditioned).
-    bool blocked_ = false, blocks_on_ = true;
+    // Blocked Krylov steps: blocked_ is set around a refined cycle none of whose slots is `stepwise`.
+    bool blocked_ = false;
     // Cholesky QR in the deflation loop: refined_ is set around refined cycles, cholqr_on_ until a factor
     // breaks down.
     bool refined_ = false, cholqr_on_ = true;
     // The cycle's systems all start from their residuals, so the residuals' coordinates in [W V] are known
     // without a pass over the basis (launch_unit_coordinates).
     bool g_direct_ = false;
-    bool cholqr_ok(int kk) const;
+    bool cholqr_ok(int kk) const;   // this cycle's deflation loop runs as Cholesky QR
     void enqueue_deflation_cholqr(int kk, long *matvecs);
     bool blocked_ok(int kk, int nsys) const;
     int enqueue_krylov_blocked(int kk, int nsys, double tol, long *matvecs);

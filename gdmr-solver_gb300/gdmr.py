@@ -55,6 +55,7 @@ SIGNATURES = {
     "solveLS_z": (D, [I, D, I, P]),
     "linOptLS_z": (None, []),
     "gdmrKernelLaunches": (LL, []),
+    "gdmrCycleCounts": (None, [P]),
     "gdmrProfile": (None, [I]),
     "gdmrProfileReset": (None, []),
     "gdmrProfileRead": (I, [I, P, P, P]),
@@ -153,6 +154,14 @@ KERNEL_CLASSES = ["projection", "update", "operator", "combine", "deflation_upda
 
 def kernel_launches() -> int:
     return int(load().gdmrKernelLaunches())
+
+
+def cycle_counts() -> dict:
+    """gdmrCycleCounts: the batched complex64 form's blocked cycles, those dropped, its deflation loops by
+    Cholesky QR and those whose factor failed, since load."""
+    c = np.zeros(4, np.int64)
+    load().gdmrCycleCounts(_ptr(c))
+    return dict(zip(("blocked", "dropped", "factored", "factor_failed"), (int(v) for v in c)))
 
 
 def profile(on: bool) -> None:

@@ -103,6 +103,11 @@ int gdmrLastHistory(gdmr_cycle *out, int max);
  * w - [W V] c, 2 operator products, 3 cycle-end combinations, 4 deflation
  * update, 5 FP64 true residual, 6 least squares, 7 SVD, 8 other. */
 long long gdmrKernelLaunches(void);
+/* Counts since load, of the batched complex64 form: counts[0] systems' cycles whose Krylov loop ran in
+ * blocks of three steps, [1] those of them whose correction was dropped because a block was
+ * ill-conditioned (the system goes on step by step), [2] deflation loops run as Cholesky QR, [3] those of
+ * them whose factor broke down (every system loses that cycle). */
+void gdmrCycleCounts(long long counts[4]);
 /* Bounded mbarrier waits (tensor-core and bulk-copy pipelines) that ran out since load: every
  * such wait gives up after about two seconds and the kernel returns with its results unset, so
  * a nonzero count means a result of this process is not to be trusted. */

@@ -28,10 +28,23 @@ def _rhs(n, nrhs, seed=50):
     return np.stack([problems.unit_gaussian_rhs(n, seed + i) for i in range(nrhs)])
 
 
+def _spread(n):
+    """A diagonal operator of 997 eigenvalues over a factor of 200, far enough from zero that no step of an
+    exhausted space falls below the absolute breakdown threshold, and a unit vector that sees two of them."""
+    i = np.arange(n) % 997
+    b = np.where((i == 0) | (i == 500), problems.unit_gaussian_rhs(n, 7), 0.0)
+    return _diagonal(2.0 ** 13 * (1 + 0.05j) * 200.0 ** (i / 996.0)), b / np.linalg.norm(b)
+
+
+def _counts(before=None):
+    c = gdmr.cycle_counts()
+    return c if before is None else {k: c[k] - before[k] for k in c}
+
+
 def _check(A, B, X, stats):
     for b, x, st in zip(B, X, stats):
         assert st["status"] == 0, st
-        assert np.linalg.norm(b - A.data * x) <= (TOL + 1e-12) * np.linalg.norm(b)
+        assert np.linalg.norm(b - A.to_scipy() @ x) <= (TOL + 1e-12) * np.linalg.norm(b)
 
 
 @pytest.mark.parametrize("nrhs", [1, 2, 8])
@@ -90,3 +103,42 @@ def test_factor_that_failed_in_an_unused_loop_is_forgotten(after):
             gdmr.multi_tail(prev)
     assert [t["status"] for t in stats] == [0, 0], stats
     s.close()
+
+
+def test_one_systems_breakdown_leaves_the_others_blocked():
+    # the first right-hand side lies in an invariant space of dimension 2: its first block is dropped, and
+    # the batch runs step by step until it has left
+    A, two = _spread(N // 3 + 41)      # three systems reach the blocked loop
+    B = np.concatenate([two[None], _rhs(A.n, 9)])
+    s = gdmr.System(A, 30, 8, capacity=4, precision="mixed")
+    alone = s.solve_batch(B[1:], tol=TOL, max_cycles=200)[1]
+    s.drop_deflation()
+    c0 = _counts()
+    X, stats = s.solve_batch(B, tol=TOL, max_cycles=200)
+    c = _counts(c0)
+    _check(A, B, X, stats)
+    assert c["dropped"] == 1, c
+    # all cycles but those beside the first system after its breakdown (three others) and those of the
+    # last one or two systems
+    beside = 4 * (stats[0]["cycles"] - 1)
+    tail = 2 * max(t["cycles"] for t in stats)
+    assert c["blocked"] >= sum(t["cycles"] for t in stats) - beside - tail > 0, (c, stats)
+    assert c["blocked"] > 4, c
+    ref, got = (np.mean([t["cycles"] for t in q]) for q in (alone, stats[1:]))
+    assert abs(got - ref) <= 1.5, (got, ref)
+    s.close()
+
+
+def test_served_requests_after_a_breakdown_run_blocked():
+    A, two = _spread(N + 1)
+    srv = gdmr.Server(budget_bytes=8 << 30)
+    op = srv.add_operator(A, 30, 8, capacity=1, precision="mixed")
+    srv.start()
+    for b, dropped in ((two, 1), (_rhs(A.n, 1)[0], 0)):
+        c0 = _counts()
+        x, st = srv.wait(srv.submit(op, b, tol=TOL), timeout=120)
+        _check(A, [b], [x], [st])
+        c = _counts(c0)
+        assert c["dropped"] == dropped, c
+    assert c["blocked"] == st["cycles"] > 0, (c, st)
+    srv.close()
