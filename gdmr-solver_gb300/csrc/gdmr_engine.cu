@@ -782,7 +782,7 @@ template <class R> void Engine<R>::enqueue_deflation_loop(int kk, long *matvecs)
 // 884,736.  Z holds approximate singular vectors, so the columns of A Z are nearly orthogonal.
 template <class R> bool Engine<R>::cholqr_ok(int kk) const {
     if constexpr (!std::is_same<R, float>::value) return false;
-    return refined_ && cholqr_on_ && kk <= CHOLQR_MAX && wapply_tc_ok(n_, kk, kk) &&
+    return refined_ && cholqr_wait_ == 0 && kk <= CHOLQR_MAX && wapply_tc_ok(n_, kk, kk) &&
            (op.kind == Operator<R>::SELL || op.kind == Operator<R>::STENCIL) &&
            (size_t)kk * kk * 2 * (((size_t)n_ + 2047) / 2048) <= scratch_size(partials_);
 }
@@ -1093,7 +1093,8 @@ template <class R> int Engine<R>::refine_setup(const SellMatrix &A64) {
     slot_.assign(cap_, Slot());
     act_h_.clear();
     kk_prev_ = 0;
-    cholqr_on_ = true;
+    cholqr_wait_ = 0;
+    cholqr_pause_ = CHOLQR_PAUSE;
     GDMR_CK(cudaMemsetAsync(X_, 0, sizeof(C) * (size_t)n_ * cap_, stream));
     return begin_solve();
 }
@@ -1257,9 +1258,11 @@ template <class R> int Engine<R>::refine_cycle(std::vector<int> *done) {
     launch_refine_update<R>(n, x64_, n, X_, n, act_, na, state_, cap_, stream);
     if (read_state(cap_ + 1) != GDMR_OK) return GDMR_ECUDA;
     const bool factor_failed = hstate_[cap_].ill != 0;   // the deflation loop's: no system has a cycle
+    if (cholqr_wait_ > 0) --cholqr_wait_;
     if (factor_failed) {
         ++g_cycle_counts[CC_FACTOR_FAILED];
-        cholqr_on_ = false;
+        cholqr_wait_ = cholqr_pause_;
+        cholqr_pause_ = std::min(2 * cholqr_pause_, CHOLQR_PAUSE_MAX);
         GDMR_CK(cudaMemsetAsync(&state_[cap_].ill, 0, sizeof(int), stream));
     }
     if (factor_failed || hstate_[lead].ill) {

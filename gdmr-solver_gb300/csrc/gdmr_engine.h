@@ -279,9 +279,13 @@ template <class R> class Engine {
     int enqueue_back(int kk, int nsys, bool join);
     // Blocked Krylov steps: blocked_ is set around a refined cycle none of whose slots is `stepwise`.
     bool blocked_ = false;
-    // Cholesky QR in the deflation loop: refined_ is set around refined cycles, cholqr_on_ until a factor
-    // breaks down.
-    bool refined_ = false, cholqr_on_ = true;
+    // Cholesky QR in the deflation loop: refined_ is set around refined cycles.  A factor that breaks down
+    // costs its cycle and pauses the form for CHOLQR_PAUSE cycles, whose updates replace the space, and for
+    // twice as long each time it happens again in a solve, CHOLQR_PAUSE_MAX at most: a space that stays
+    // singular costs one cycle in 65, an accident no more than a few cycles of the loop.
+    static constexpr int CHOLQR_PAUSE = 4, CHOLQR_PAUSE_MAX = 64;
+    bool refined_ = false;
+    int cholqr_wait_ = 0, cholqr_pause_ = CHOLQR_PAUSE;
     // The cycle's systems all start from their residuals, so the residuals' coordinates in [W V] are known
     // without a pass over the basis (launch_unit_coordinates).
     bool g_direct_ = false;

@@ -124,6 +124,7 @@ def test_one_systems_breakdown_leaves_the_others_blocked():
     tail = 2 * max(t["cycles"] for t in stats)
     assert c["blocked"] >= sum(t["cycles"] for t in stats) - beside - tail > 0, (c, stats)
     assert c["blocked"] > 4, c
+    assert c["factored"] > c["factor_failed"], c
     ref, got = (np.mean([t["cycles"] for t in q]) for q in (alone, stats[1:]))
     assert abs(got - ref) <= 1.5, (got, ref)
     s.close()
@@ -142,3 +143,19 @@ def test_served_requests_after_a_breakdown_run_blocked():
         assert c["dropped"] == dropped, c
     assert c["blocked"] == st["cycles"] > 0, (c, st)
     srv.close()
+
+
+def test_cholesky_factor_returns_after_a_failure():
+    A = problems.helmholtz((20, 19, 18), 8.0, 0.05)
+    Z = _rhs(A.n, 8, 900)
+    Z[5] = Z[2]
+    s = gdmr.System(A, 20, 8, capacity=1, precision="mixed")
+    s.import_deflation(Z)
+    c0 = _counts()
+    X, stats = s.solve_batch(_rhs(A.n, 1), tol=TOL, max_cycles=400)
+    c = _counts(c0)
+    _check(A, _rhs(A.n, 1), X, stats)
+    # the failed cycle, four without, then every one
+    assert stats[0]["cycles"] > 8 and c["factor_failed"] == 1, (c, stats)
+    assert c["factored"] == stats[0]["cycles"] - 4, (c, stats)
+    s.close()
