@@ -543,6 +543,64 @@ extern "C" int gdmr_shared_basis_check(int n, int k, int nsys, const float *W_ri
     return GDMR_OK;
 }
 
+// The orthonormalisation of the refined complex64 cycles' deflation loop (W = orth(A Z)) on its own.
+extern "C" int gdmr_orthonormalise_check(int n, int k, const float *A_ri, float *W_ri, double *R_ri, int *failed) {
+    const char *F = "gdmr_orthonormalise_check";
+    if (n < 1 || k < 8 || k > CHOLQR_MAX || !wapply_tc_ok(n, k, k))
+        return fail(GDMR_EINVAL, F, "need n >= 1 and 8 <= k <= 32");
+    if (!A_ri || !W_ri || !R_ri || !failed) return fail(GDMR_EINVAL, F, "null buffer");
+    float2 *Wd = nullptr, *Td = nullptr;
+    double2 *gram = nullptr, *r = nullptr, *hd = nullptr, *part = nullptr;
+    unsigned *tickets = nullptr;
+    SysState *state = nullptr;
+    int *act = nullptr;
+    const size_t wb = sizeof(float2) * (size_t)k * n, kb = sizeof(double2) * k * k, scratch = scratch_doubles(k, k, n);
+    auto release = [&]() {
+        if (part) unregister_scratch(part);
+        cudaFree(Wd);
+        cudaFree(Td);
+        cudaFree(gram);
+        cudaFree(r);
+        cudaFree(hd);
+        cudaFree(part);
+        cudaFree(tickets);
+        cudaFree(state);
+        cudaFree(act);
+    };
+    if (cudaMalloc(&Wd, wb) != cudaSuccess || cudaMalloc(&Td, wb) != cudaSuccess || cudaMalloc(&gram, kb) != cudaSuccess ||
+        cudaMalloc(&r, 2 * kb) != cudaSuccess || cudaMalloc(&hd, kb) != cudaSuccess ||
+        cudaMalloc(&part, sizeof(double) * scratch) != cudaSuccess ||
+        cudaMalloc(&tickets, sizeof(unsigned) * k) != cudaSuccess || cudaMalloc(&state, sizeof(SysState)) != cudaSuccess ||
+        cudaMalloc(&act, sizeof(int) * k) != cudaSuccess) {
+        release();
+        return fail(GDMR_ENOMEM, F, "device allocation failed");
+    }
+    register_scratch(part, scratch);
+    std::vector<int> ident(k);
+    for (int i = 0; i < k; ++i) ident[i] = i;
+    SysState hs{};
+    cudaError_t e = cudaMemcpy(Wd, A_ri, wb, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(act, ident.data(), sizeof(int) * k, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemset(tickets, 0, sizeof(unsigned) * k);
+    if (e == cudaSuccess) e = cudaMemset(state, 0, sizeof(SysState));
+    if (e == cudaSuccess) e = cudaMemset(hd, 0, kb);
+    if (e == cudaSuccess && push_wait_limit() != 0) e = cudaErrorUnknown;
+    const unsigned t0 = wproj_tc_timeouts();
+    if (e == cudaSuccess) {
+        launch_orthonormalise(n, k, Wd, Td, act, part, tickets, gram, k, r, hd, k, state, 0);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = cudaMemcpy(W_ri, Wd, wb, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(R_ri, hd, kb, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(&hs, state, sizeof hs, cudaMemcpyDeviceToHost);
+    release();
+    if (e != cudaSuccess) return fail(GDMR_ECUDA, F, cudaGetErrorString(e));
+    if (wproj_tc_timeouts() != t0) return fail(GDMR_ETIMEOUT, F, "a pipeline wait ran out");
+    *failed = hs.ill != 0;
+    return GDMR_OK;
+}
+
 // ================================================================ context API
 // complex128 <-> complex64 helpers used by the context API
 namespace {

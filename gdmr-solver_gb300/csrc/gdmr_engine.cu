@@ -793,15 +793,8 @@ template <class R> void Engine<R>::enqueue_deflation_cholqr(int kk, long *matvec
         if (op.kind == Operator<R>::SELL) launch_spmm<R>(op.sell, Z_, n, W_, n, ident_, kk, stream);
         else launch_stencil<R>(op.stencil, Z_, n, W_, n, ident_, kk, stream);
         // vs_, svdwork_ and Znew_ are the deflation update's, joined before this loop
-        double2 *r1 = svdwork_, *r2 = svdwork_ + kk * kk;
-        for (int pass = 0; pass < 2; ++pass) {
-            const C *in = pass ? Znew_ : W_;
-            launch_mdot<R>(n, in, kk, nullptr, 0, 0, in, n, ident_, kk, partials_, kk, tickets_ + cap_ + 1, vs_, m, state_, false,
-                           stream);
-            launch_cholqr(kk, vs_, m, pass ? r2 : r1, pass ? r1 : nullptr, Hd_, m + 1, state_ + cap_, stream);
-            ProfScope p(KC_UPDATE, sizeof(C) * 2.0 * kk * n, stream, 1);
-            launch_wapply_tc(n, kk, in, vs_, m, ident_, kk, pass ? W_ : Znew_, n, -1, stream);
-        }
+        launch_orthonormalise(n, kk, W_, Znew_, ident_, partials_, tickets_ + cap_ + 1, vs_, m, svdwork_, Hd_, m + 1,
+                              state_ + cap_, stream);
     }
 }
 

@@ -5643,6 +5643,26 @@ void launch_cholqr(int k, double2 *gram, int ldg, double2 *r, const double2 *r1,
     k_cholqr<<<1, dim3(CHOLQR_MAX, CHOLQR_MAX), 0, stream>>>(k, gram, ldg, r, r1, hd, ldh, st);
 }
 
+// The Gram matrices are summed by k_wdots (k_mdot where its partial sums do not fit), never on the tensor
+// cores, whatever the tuner would pick: an accumulator there takes a few hundred truncated additions, which
+// are all one way on the diagonal.  For 24 Gaussian vectors the norms came out off by 1.9e-5 at n = 884,736
+// and 4.7e-6 at 262,144 (2e-9 here), and W with them; the loop over the vectors had no such error.
+void launch_orthonormalise(int n, int k, float2 *W, float2 *T, const int *ident, double2 *partials, unsigned *tickets,
+                           double2 *gram, int ldg, double2 *r, double2 *hd, int ldh, SysState *st, cudaStream_t stream) {
+    for (int pass = 0; pass < 2; ++pass) {
+        const float2 *in = pass ? T : W;
+        {
+            Launch L_(KC_MDOT, (double)sizeof(float2) * n * 2.0 * k, stream, 2);
+            if (!wdots_run(n, k, in, in, n, ident, k, partials, scratch_capacity(partials), gram, ldg, stream))
+                mdot_dispatch<float>(0, n, in, k, nullptr, 0, 0, in, n, ident, k, partials, k, tickets, gram, ldg, nullptr,
+                                     false, stream);
+        }
+        launch_cholqr(k, gram, ldg, pass ? r + k * k : r, pass ? r : nullptr, hd, ldh, st, stream);
+        Launch L_(KC_UPDATE, (double)sizeof(float2) * 2.0 * k * n, stream, 1);
+        launch_wapply_tc(n, k, in, gram, ldg, ident, k, pass ? W : T, n, -1, stream);
+    }
+}
+
 void launch_wdeflate(int n, int kk, const float2 *W, const float2 *y, size_t strideY, float2 *out, size_t strideO,
                      const int *act, int nsys, double2 *coef, size_t strideC, double2 *partials, int qmax,
                      unsigned *tickets, SysState *state, cudaStream_t st) {

@@ -280,12 +280,16 @@ int launch_wupdate_tc(int n, int kk, const float2 *W, const float2 *V, size_t st
 void launch_wdeflate(int n, int kk, const float2 *W, const float2 *y, size_t strideY, float2 *out, size_t strideO,
                      const int *act, int nsys, double2 *coef, size_t strideC, double2 *partials, int qmax,
                      unsigned *tickets, SysState *state, cudaStream_t st);
-// One pass of the deflation loop's Cholesky QR (complex64 vectors): from the Gram matrix gram[i*ldg + l] =
-// <a_l, a_i> of k <= 32 vectors, the factor R (R^H R = G) into r (k x k, column-major) and R^-1 in
-// place of gram: column i at gram + i*ldg.  With r1, the factor of the pass before, R r1 goes to hd
-// (leading dimension ldh), the deflation block of the Hessenberg.  A pivot below 1e-3 of its column
-// makes the results zero and sets st->ill (of the shared pseudo-system) to 2; the first pass (r1 null)
-// clears it otherwise.
+// W <- orth(W) for k complex64 vectors of n by two passes of Cholesky QR, T a second array of them; the
+// factor R (W_in = W_out R) goes to the upper triangle of hd (leading dimension ldh).  Needs
+// wapply_tc_ok(n, k, k) and k <= CHOLQR_MAX; gram: k columns of leading dimension ldg >= k; r: 2 k^2;
+// ident: 0..k-1; tickets: k.  A pivot below 1e-3 of its column makes the results zero and sets st->ill
+// (of the shared pseudo-system) to 2, which the first pass clears otherwise.
+void launch_orthonormalise(int n, int k, float2 *W, float2 *T, const int *ident, double2 *partials, unsigned *tickets,
+                           double2 *gram, int ldg, double2 *r, double2 *hd, int ldh, SysState *st, cudaStream_t stream);
+// One pass's factor: from the Gram matrix gram[i*ldg + l] = <a_l, a_i>, R (R^H R = G) into r (k x k,
+// column-major) and R^-1 in place of gram: column i at gram + i*ldg.  With r1, the factor of the pass
+// before, R r1 goes to hd.
 constexpr int CHOLQR_MAX = 32;
 void launch_cholqr(int k, double2 *gram, int ldg, double2 *r, const double2 *r1, double2 *hd, int ldh, SysState *st,
                    cudaStream_t stream);

@@ -70,6 +70,7 @@ SIGNATURES = {
     "gdmrAsyncTimeouts": (ctypes.c_uint, []),
     "gdmr_hessenberg_svd": (I, [I, I, P, P, P, P]),
     "gdmr_shared_basis_check": (I, [I, I, I, P, P, P, P, P]),
+    "gdmr_orthonormalise_check": (I, [I, I, P, P, P, P]),
     "gdmr_system_set_stencil": (I, [P, I, I, I, P]),
     "gdmr_system_clear_stencil": (I, [P]),
     "gdmr_system_create": (I, [P, I, P, P, P, I, I, I, I, I]),
@@ -260,6 +261,17 @@ def shared_basis_check(W, Y, c):
     _check(load().gdmr_shared_basis_check(n, k, nsys, _ptr(W), _ptr(Y), _ptr(c), _ptr(coef), _ptr(P)),
            "gdmr_shared_basis_check")
     return coef, P
+
+
+def orthonormalise_check(A):
+    """The deflation loop's Cholesky QR on its own (gdmr_orthonormalise_check): A (k, n) complex64; returns
+    (W, R, failed) with W (k, n) complex64, R (k, k) complex128 upper triangular and A = R^T W."""
+    A = np.ascontiguousarray(A, dtype=np.complex64)
+    k, n = A.shape
+    W, R, failed = np.empty_like(A), np.empty((k, k), np.complex128), ctypes.c_int(0)
+    _check(load().gdmr_orthonormalise_check(n, k, _ptr(A), _ptr(W), _ptr(R), ctypes.byref(failed)),
+           "gdmr_orthonormalise_check")
+    return W, R.T.copy(), bool(failed.value)
 
 
 def profile_read() -> dict:

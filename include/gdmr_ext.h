@@ -145,6 +145,12 @@ int gdmr_hessenberg_svd(int m, int k, const double *H, double *sigma, double *vs
  * otherwise).  Allocates its own device buffers and synchronises the device. */
 int gdmr_shared_basis_check(int n, int k, int nsys, const float *W, const float *Y, const double *c, double *coef,
                             float *P);
+/* The orthonormalisation W = orth(A) of the batched complex64 form's deflation loop on its own, run once on
+ * host data: two passes of Cholesky QR.  A, W: k x n complex64 (vectors contiguous); R: k x k complex128,
+ * column-major, the upper triangular factor (A_j = sum_i R_ij W_i); *failed <- 1 (and zeros) if a pivot
+ * falls below 1e-3 of its column's squared norm, else 0.  n >= 1, 8 <= k <= 32 (GDMR_EINVAL otherwise).
+ * Allocates its own device buffers and synchronises the device. */
+int gdmr_orthonormalise_check(int n, int k, const float *A, float *W, double *R, int *failed);
 /* Gram-Schmidt kernel autotuning: the first launch of a shape times the kernel variants
  * and keeps the fastest for the process (on by default; off selects the first variant).
  * The report lists one line per tuned shape with the time of every variant. */
