@@ -543,6 +543,59 @@ extern "C" int gdmr_shared_basis_check(int n, int k, int nsys, const float *W_ri
     return GDMR_OK;
 }
 
+// The projection launcher of the complex64 cycles on its own: the tuner's variant, or the forced one.
+extern "C" int gdmr_projection_check(int n, int k, int nsys, const float *W_ri, const float *Y_ri, double *coef_ri) {
+    const char *F = "gdmr_projection_check";
+    if (n < 1 || k < 1 || k > 160 || nsys < 1 || nsys > 65535)
+        return fail(GDMR_EINVAL, F, "need n >= 1, 1 <= k <= 160 and 1 <= nsys <= 65535");
+    if (!W_ri || !Y_ri || !coef_ri) return fail(GDMR_EINVAL, F, "null buffer");
+    float2 *Wd = nullptr, *Yd = nullptr;
+    double2 *coef = nullptr, *part = nullptr;
+    unsigned *tickets = nullptr;
+    SysState *state = nullptr;
+    int *act = nullptr;
+    const size_t wb = sizeof(float2) * (size_t)k * n, yb = sizeof(float2) * (size_t)nsys * n;
+    const size_t cb = sizeof(double2) * (size_t)k * nsys, scratch = scratch_doubles(k, nsys, n);
+    auto release = [&]() {
+        if (part) unregister_scratch(part);
+        cudaFree(Wd);
+        cudaFree(Yd);
+        cudaFree(coef);
+        cudaFree(part);
+        cudaFree(tickets);
+        cudaFree(state);
+        cudaFree(act);
+    };
+    if (cudaMalloc(&Wd, wb) != cudaSuccess || cudaMalloc(&Yd, yb) != cudaSuccess || cudaMalloc(&coef, cb) != cudaSuccess ||
+        cudaMalloc(&part, sizeof(double) * scratch) != cudaSuccess ||
+        cudaMalloc(&tickets, sizeof(unsigned) * nsys) != cudaSuccess ||
+        cudaMalloc(&state, sizeof(SysState) * nsys) != cudaSuccess || cudaMalloc(&act, sizeof(int) * nsys) != cudaSuccess) {
+        release();
+        return fail(GDMR_ENOMEM, F, "device allocation failed");
+    }
+    register_scratch(part, scratch);
+    std::vector<int> ident(nsys);
+    for (int i = 0; i < nsys; ++i) ident[i] = i;
+    cudaError_t e = cudaMemcpy(Wd, W_ri, wb, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(Yd, Y_ri, yb, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(act, ident.data(), sizeof(int) * nsys, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemset(tickets, 0, sizeof(unsigned) * nsys);
+    if (e == cudaSuccess) e = cudaMemset(state, 0, sizeof(SysState) * nsys);
+    if (e == cudaSuccess && push_wait_limit() != 0) e = cudaErrorUnknown;
+    const unsigned t0 = wproj_tc_timeouts();
+    if (e == cudaSuccess) {
+        launch_mdot<float>(n, Wd, k, nullptr, 0, 0, Yd, (size_t)n, act, nsys, part, k, tickets, coef, (size_t)k, state, false,
+                           0);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = cudaMemcpy(coef_ri, coef, cb, cudaMemcpyDeviceToHost);
+    release();
+    if (e != cudaSuccess) return fail(GDMR_ECUDA, F, cudaGetErrorString(e));
+    if (wproj_tc_timeouts() != t0) return fail(GDMR_ETIMEOUT, F, "a pipeline wait ran out");
+    return GDMR_OK;
+}
+
 // The orthonormalisation of the refined complex64 cycles' deflation loop (W = orth(A Z)) on its own.
 extern "C" int gdmr_orthonormalise_check(int n, int k, const float *A_ri, float *W_ri, double *R_ri, int *failed) {
     const char *F = "gdmr_orthonormalise_check";

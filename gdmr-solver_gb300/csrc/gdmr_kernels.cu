@@ -1757,9 +1757,12 @@ __global__ void __launch_bounds__(NT) k_wproj_reduce(int kk, int nsys, int G, co
 // systems (blockIdx.y).  Chunks of WD_CH rows of W and of the group's y come in by cp.async, WD_ST deep;
 // lanes are rows, and each of the 24 warps holds one tile of 4 x 4 outputs in registers for all its rows,
 // so a row's 4 + 4 values feed 16 complex products.  With 12 or 6 tiles or fewer, RS = 2 or 4 warps
-// share a tile, each on every RS-th group of 32 rows.  FP32 chains of WD_CHAIN products at most,
-// then the warp's tree, then double-float over the CTAs (k_wdots_reduce).
-constexpr int WD_CH = 128, WD_ST = 3, WD_CHAIN = 128, WD_KMAX = 32, WD_WARPS = 24, WD_NT = WD_WARPS * 32;
+// share a tile, each on every RS-th group of 32 rows.  As in k_mdot, no FP32 sum holds more than 256
+// products: a lane's chains of WD_CHAIN = 8, then the warp's tree; double-float from there on.  The trees
+// cost a tenth to a sixth where a launch is short: n = 262,144, kk = 24, 16 systems 41.5 us against 36.9
+// with chains of 128 and one tree at the end (sums off by up to 1.9e-6 of their terms, here by 1.2e-7).
+// One wave of CTAs, which chains that long could not always keep, pays for them at n = 884,736: 114 us (132).
+constexpr int WD_CH = 128, WD_ST = 3, WD_CHAIN = 8, WD_KMAX = 32, WD_WARPS = 24, WD_NT = WD_WARPS * 32;
 __device__ __forceinline__ void cp_async16z(void *dst, const void *src, int bytes) {   // zero-filled past `bytes`
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
                  "l"(src), "r"(bytes));
@@ -1814,6 +1817,8 @@ __global__ void __launch_bounds__(WD_NT, 1) k_wdots(int n, int kk, const float2 
         wo[a] = min(p0 + a, kk - 1) * WD_CH + rs * 32 + lane;
         yo[a] = (kk + min(c0 + a, ns - 1)) * WD_CH + rs * 32 + lane;
     }
+    dfr sum(0.f, 0.f);                                    // component `lane` = 8 a + 2 c + (re | im) of the tile
+    constexpr int FLUSH = WD_CHAIN * 32 * RS / WD_CH;     // chunks whose rows make WD_CHAIN products a lane
     for (int ch = 0; ch < WD_ST - 1; ++ch) issue(ch);
     for (int ch = 0; ch < nch; ++ch) {
         asm volatile("cp.async.wait_group %0;\n" ::"n"(WD_ST - 2) : "memory");
@@ -1836,31 +1841,35 @@ __global__ void __launch_bounds__(WD_NT, 1) k_wdots(int n, int kk, const float2 
                         for (int c = 0; c < 4; ++c) cdotacc(acc[a][c], w[a], y[c]);
                 }
             }
+            if ((ch + 1) % FLUSH == 0 || ch + 1 == nch) {
+                // reduce-scatter of the 32 sums over the warp: lane l ends with component l
+                float v[32];
+#pragma unroll
+                for (int a = 0; a < 4; ++a)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        v[8 * a + 2 * c] = acc[a][c].x;
+                        v[8 * a + 2 * c + 1] = acc[a][c].y;
+                        acc[a][c] = make_float2(0.f, 0.f);
+                    }
+#pragma unroll
+                for (int half = 16; half > 0; half >>= 1) {
+                    const bool hi = lane & half;
+#pragma unroll
+                    for (int q = 0; q < half; ++q) {
+                        const float keep = hi ? v[half + q] : v[q], send = hi ? v[q] : v[half + q];
+                        v[q] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+                    }
+                }
+                sum = sum + dfr(v[0], 0.f);
+            }
         }
     }
     if (!busy) return;
-    // reduce-scatter of the 32 sums over the warp: lane l ends with component l = 8 a + 2 c + (re | im)
-    float v[32];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            v[8 * a + 2 * c] = acc[a][c].x;
-            v[8 * a + 2 * c + 1] = acc[a][c].y;
-        }
-#pragma unroll
-    for (int half = 16; half > 0; half >>= 1) {
-        const bool hi = lane & half;
-#pragma unroll
-        for (int q = 0; q < half; ++q) {
-            const float keep = hi ? v[half + q] : v[q], send = hi ? v[q] : v[half + q];
-            v[q] = keep + __shfl_xor_sync(0xffffffffu, send, half);
-        }
-    }
     const int Gt = gridDim.x * RS, g = blockIdx.x * RS + rs;
     const int p = p0 + (lane >> 3), c = c0 + ((lane >> 1) & 3);
     if (p < kk && c < ns)
-        store_df(part + (((size_t)p * nsys + s0 + c) * 2 + (lane & 1)) * Gt + g, dfr(v[0], 0.f));
+        store_df(part + (((size_t)p * nsys + s0 + c) * 2 + (lane & 1)) * Gt + g, sum);
 }
 // coef_s[p] = the sum over the Gt partials of output (p, s): one warp an output, fixed order.
 __global__ void __launch_bounds__(NT) k_wdots_reduce(int kk, int nsys, int Gt, const double *__restrict__ part,
@@ -5045,7 +5054,7 @@ int bucket_of(int nsys, int qa, int qb) {
     // a batch against the shared vectors alone (the deflator of the blocked Krylov steps, the deflation
     // loop's Gram matrix): classes of its own by the batch, since the tensor cores' share of the time
     // hardly grows with it (at n = 884,736, kk = 24: 173 us for 16 systems, 211 for 64) and the CUDA
-    // cores' does (130 and 367 us)
+    // cores' does (114 and 407 us)
     const int wide = nsys < 8 ? 0 : nsys <= 16 ? 1 : nsys <= 32 ? 2 : 3;
     return (nsys > 1 ? 1 : 0) + (qa > 0 ? 2 : 0) + (nsys > 1 && qa > 0 && qb == 0 ? 4 + 8 * wide : 0);
 }
@@ -5235,8 +5244,7 @@ bool wdots_run(int n, int kk, const float2 *W, const float2 *Y, size_t strideY, 
     const int tiles = tilesP * ((sg + 3) / 4);
     const int RS = tiles > 12 ? 1 : tiles > 6 ? 2 : 4;
     const int nch = (n + WD_CH - 1) / WD_CH, groups = (nsys + sg - 1) / sg;
-    // one CTA an SM over the groups, or more where a lane's FP32 chain would pass WD_CHAIN products
-    const int G = std::min(nch, std::max((num_sms() + groups - 1) / groups, (nch * (WD_CH / 32) + WD_CHAIN * RS - 1) / (WD_CHAIN * RS)));
+    const int G = std::min(nch, std::max(num_sms() / groups, 1));   // one wave of one CTA an SM over the groups
     if ((size_t)kk * nsys * 2 * RS * G > cap) return false;
     const int vec2 = n % 2 == 0 && strideY % 2 == 0 && ((uintptr_t)W & 15) == 0 && ((uintptr_t)Y & 15) == 0;
     const size_t smem = (size_t)WD_ST * (kk + sg) * WD_CH * sizeof(float2);

@@ -70,6 +70,7 @@ SIGNATURES = {
     "gdmrAsyncTimeouts": (ctypes.c_uint, []),
     "gdmr_hessenberg_svd": (I, [I, I, P, P, P, P]),
     "gdmr_shared_basis_check": (I, [I, I, I, P, P, P, P, P]),
+    "gdmr_projection_check": (I, [I, I, I, P, P, P]),
     "gdmr_orthonormalise_check": (I, [I, I, P, P, P, P]),
     "gdmr_system_set_stencil": (I, [P, I, I, I, P]),
     "gdmr_system_clear_stencil": (I, [P]),
@@ -261,6 +262,17 @@ def shared_basis_check(W, Y, c):
     _check(load().gdmr_shared_basis_check(n, k, nsys, _ptr(W), _ptr(Y), _ptr(c), _ptr(coef), _ptr(P)),
            "gdmr_shared_basis_check")
     return coef, P
+
+
+def projection_check(W, Y):
+    """The complex64 projection on its own (gdmr_projection_check), with the tuner's variant or the one pinned
+    by tune_force: W (k, n), Y (nsys, n) complex64; returns (nsys, k) complex128 <W_p, Y_s>."""
+    W = np.ascontiguousarray(W, dtype=np.complex64)
+    Y = np.ascontiguousarray(Y, dtype=np.complex64)
+    coef = np.empty((Y.shape[0], W.shape[0]), np.complex128)
+    _check(load().gdmr_projection_check(W.shape[1], W.shape[0], Y.shape[0], _ptr(W), _ptr(Y), _ptr(coef)),
+           "gdmr_projection_check")
+    return coef
 
 
 def orthonormalise_check(A):

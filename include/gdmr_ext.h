@@ -145,6 +145,11 @@ int gdmr_hessenberg_svd(int m, int k, const double *H, double *sigma, double *vs
  * otherwise).  Allocates its own device buffers and synchronises the device. */
 int gdmr_shared_basis_check(int n, int k, int nsys, const float *W, const float *Y, const double *c, double *coef,
                             float *P);
+/* The complex64 projection coef[s*k + p] = <W_p, Y_s> of the restart cycles on its own, run once on host
+ * data with the variant that the tuner picks or gdmrTuneForce pins; layouts as above.  n >= 1,
+ * 1 <= k <= 160, 1 <= nsys <= 65535 (GDMR_EINVAL otherwise).  Allocates its own device buffers and
+ * synchronises the device. */
+int gdmr_projection_check(int n, int k, int nsys, const float *W, const float *Y, double *coef);
 /* The orthonormalisation W = orth(A) of the batched complex64 form's deflation loop on its own, run once on
  * host data: two passes of Cholesky QR.  A, W: k x n complex64 (vectors contiguous); R: k x k complex128,
  * column-major, the upper triangular factor (A_j = sum_i R_ij W_i); *failed <- 1 (and zeros) if a pivot
