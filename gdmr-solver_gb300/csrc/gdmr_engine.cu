@@ -661,7 +661,7 @@ template <class R> int Engine<R>::run_cycle(int kk, int nsys, int lead, double t
         long mv = 0;
         const bool hz = have_z_, zp = z_pending_;
         int rc = enqueue_cycle(kk, nsys, tol, &mv, true);
-        set_capturing(false);
+        const bool untuned = set_capturing(false);
         have_z_ = hz;
         z_pending_ = zp;
         cudaGraph_t graph = nullptr;
@@ -670,6 +670,10 @@ template <class R> int Engine<R>::run_cycle(int kk, int nsys, int lead, double t
         if (e != cudaSuccess) {
             set_last_error(GDMR_ECUDA, std::string("restart-cycle capture: ") + cudaGetErrorString(e));
             return GDMR_ECUDA;
+        }
+        if (untuned) {   // some launch's variant is not chosen yet: an eager cycle times its class
+            cudaGraphDestroy(graph);
+            return enqueue_cycle(kk, nsys, tol, matvecs, false);
         }
         e = cudaGraphInstantiate(&exec, graph, 0);
         cudaGraphDestroy(graph);
@@ -692,8 +696,8 @@ template <class R> int Engine<R>::run_cycle(int kk, int nsys, int lead, double t
 }
 
 // CUDA graphs pay off where launch overhead is comparable to the work: small n x batch.  The
-// first two cycles of an engine run eagerly: they tune the kernels of both cycle shapes
-// (without and with the deflation space) before anything is captured.
+// first two cycles of an engine run eagerly: they tune most kernels of both cycle shapes
+// (without and with the deflation space); run_cycle drops a capture that meets a class they did not.
 template <class R> bool Engine<R>::graph_ok(int nsys) const {
     return use_graphs && op.kind != Operator<R>::HOOK && !profile_enabled() && cycles_run_ > 1 &&
            (long)n_ * nsys <= (1L << 20);

@@ -5046,12 +5046,13 @@ int forced_variant(int kernel) {
     return g_forced[kernel];
 }
 thread_local bool t_capturing = false;   // a stream capture is open on this thread: no timing
+thread_local bool t_untuned = false;     // it met a class that has no variant yet
 
 // One choice per (precision, kernel, n, shape class).  The shape class separates launches
 // with and without a shared segment (the deflation vectors W) and single- from multi-system
 // launches, because a batch sharing W is limited by re-reading W and favours other tiles.
-// Engines run their first two cycles eagerly, so every class they use is settled before a
-// cycle is captured into a CUDA graph.
+// A cycle captured into a CUDA graph holds settled classes only: one that meets an unsettled class (a
+// batch that has shrunk into another width) is not kept, and the cycle runs eagerly (Engine::run_cycle).
 int bucket_of(int nsys, int qa, int qb) {
     // a batch against the shared vectors alone (the deflator of the blocked Krylov steps, the deflation
     // loop's Gram matrix): classes of its own by the batch, since the tensor cores' share of the time
@@ -5073,7 +5074,11 @@ int tuned_variant(int prec, int kernel, int n, int nsys, int qa, int qb, int nva
         std::lock_guard<std::mutex> lk(g_tune_mu);
         for (auto &e : g_tuned)
             if (e.key == key) return e.variant;
-        if (!g_tune_enabled || t_capturing) return 0;
+        if (!g_tune_enabled) return 0;
+        if (t_capturing) {
+            t_untuned = true;
+            return 0;
+        }
     }
     cudaEvent_t a, b;
     cudaEventCreate(&a);
@@ -5115,7 +5120,12 @@ int tuned_variant(int prec, int kernel, int n, int nsys, int qa, int qb, int nva
 }
 }  // namespace
 
-void set_capturing(bool on) { t_capturing = on; }
+bool set_capturing(bool on) {
+    const bool untuned = t_untuned;
+    t_capturing = on;
+    t_untuned = false;
+    return untuned;
+}
 
 void tune_force(int projection, int update) {
     std::lock_guard<std::mutex> lk(g_tune_mu);

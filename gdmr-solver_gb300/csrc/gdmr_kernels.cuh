@@ -216,8 +216,9 @@ void profile_reset();
 void tune_enable(bool on);
 // Pins the projection and update variants (-1 returns each to the tuner).
 void tune_force(int projection, int update);
-// Marks the calling thread as capturing a CUDA graph: launchers then use cached choices only.
-void set_capturing(bool on);
+// Marks the calling thread as capturing a CUDA graph: launchers then use cached choices only.  Returns whether one
+// of them has met a class without a choice since the last call.
+bool set_capturing(bool on);
 std::string tune_report();
 
 // ----------------------------------------------------------------- launchers
