@@ -5704,6 +5704,16 @@ void launch_wdeflate(int n, int kk, const float2 *W, const float2 *y, size_t str
                                    coef, strideC, partials, tickets, state, f, false, st);
     };
     int v = 0;
+    const int forced = forced_variant(1);
+    if (forced >= 0) {   // a pinned update pins the subtraction too: 9 and 10 apply W c on the tensor cores
+        if ((forced == 9 || forced == 10) && tc) {
+            run(0);
+        } else {
+            update_dispatch<float>(forced, n, W, kk, nullptr, 0, 0, y, strideY, out, strideO, act, nsys, coef, strideC,
+                                   partials, tickets, state, f, false, st);
+        }
+        return;
+    }
     if (nsys > 1 && !profile_enabled()) v = tuned_variant(prec_key<float>(), 2, n, nsys, kk, 0, 4, st, run);
     else {
         std::lock_guard<std::mutex> lk(g_tune_mu);

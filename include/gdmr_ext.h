@@ -170,7 +170,9 @@ const char *gdmrTuneReport(void);
  * into the next basis slot, then the per-system update), 10 (one kernel: the shared part on
  * the tensor cores, subtracted from TMEM while the own basis streams; at most 32 own vectors)
  * and 11 (one kernel, every system of the batch per CTA with the rows of the shared part in
- * registers; at most 128 systems); complex128 projection 7 and update 6 (CUDA cores). */
+ * registers; at most 128 systems); complex128 projection 7 and update 6 (CUDA cores).
+ * A pinned update pins the deflator's subtraction in the blocked cycles of complex64 batches too: 9 and 10
+ * the tensor-core form, the others the kernel of that index. */
 void gdmrTuneForce(int projectionVariant, int updateVariant);
 
 /* Structured-grid operator kernel (on by default).  A CSR matrix whose non-zeros all lie on the
