@@ -5834,12 +5834,12 @@ void launch_svd_smallest(int m, int k, const double2 *H, size_t strideH, const i
     if (use_smem) allow_smem(k_svd<false>, smem);
     const int pairs = (m + 1) / 2;
     const int threads = 32 * (pairs < 32 ? (pairs > 4 ? pairs : 4) : 32);
-    // 40 to 63 columns: a cluster of 4 CTAs up to 24 pairs, 8 above, where the exchange buffers fit beside the
-    // work.  In clocks, one CTA against the cluster: m = 30, k = 8: 578 to 650 thousand; m = 40, k = 10: 1070 to
-    // 1028; m = 48, k = 24: 1717 to 1355; m = 60, k = 20: 2430 to 1755 (below, a round is one pair's latency)
-    const int nc = m < 40 || m > 63 ? 1 : pairs <= 24 ? 4 : 8, wpc = (pairs + nc - 1) / nc;
-    const size_t exch = sizeof(dfc) * 4 * (size_t)wpc * (2 * m + 2);
-    if (nc > 1 && smem + exch <= 220 * 1024) {
+    // 40 to 62 columns: a cluster of 4 CTAs up to 24 pairs, 8 above; beyond, the exchange buffers no longer fit
+    // beside the work.  In clocks, one CTA against the cluster: m = 30, k = 8: 578 to 650 thousand; m = 40, k = 10:
+    // 1070 to 1028; m = 48, k = 24: 1717 to 1355; m = 60, k = 20: 2430 to 1755 (below, a round is one pair's latency)
+    const int nc = m < 40 || m > 62 ? 1 : pairs <= 24 ? 4 : 8, wpc = (pairs + nc - 1) / nc;
+    if (nc > 1) {
+        const size_t exch = sizeof(dfc) * 4 * (size_t)wpc * (2 * m + 2);   // 219,744 bytes with the work at m = 62
         allow_smem(k_svd<true>, smem + exch);
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(nc);
@@ -5852,8 +5852,8 @@ void launch_svd_smallest(int m, int k, const double2 *H, size_t strideH, const i
         at.val.clusterDim.y = at.val.clusterDim.z = 1;
         cfg.attrs = &at;
         cfg.numAttrs = 1;
-        cudaLaunchKernelEx(&cfg, k_svd<true>, m, k, H, strideH, lead, vs, sigma, work, 1, sweeps);
-        return;
+        if (cudaLaunchKernelEx(&cfg, k_svd<true>, m, k, H, strideH, lead, vs, sigma, work, 1, sweeps) == cudaSuccess) return;
+        cudaGetLastError();   // refused (no room for a cluster): one CTA
     }
     k_svd<false><<<1, threads, use_smem ? smem : 0, st>>>(m, k, H, strideH, lead, vs, sigma, work, use_smem, sweeps);
 }
