@@ -647,10 +647,20 @@ template <class R> int Engine<R>::run_cycle(int kk, int nsys, int lead, double t
     const int zpar = zpar_;
     const bool blocked = blocked_ok(kk, nsys), cholqr = cholqr_ok(kk);
     cudaGraphExec_t exec = nullptr;
-    for (auto &g : graphs_)
-        if (g.kk == kk && g.nsys == nsys && g.zpar == zpar && g.tol == tol && g.blocked == blocked &&
-            g.cholqr == cholqr && g.gdirect == g_direct_)
+    const int generation = tune_generation(n_);
+    for (size_t i = 0; i < graphs_.size(); ++i) {
+        const GraphEntry &g = graphs_[i];
+        if (g.kk != kk || g.nsys != nsys || g.zpar != zpar || g.tol != tol || g.blocked != blocked ||
+            g.cholqr != cholqr || g.gdirect != g_direct_)
+            continue;
+        if (g.generation >= 0 && g.generation != generation) {   // captured before a class was settled
+            cudaGraphExecDestroy(g.exec);
+            graphs_.erase(graphs_.begin() + i);
+        } else {
             exec = g.exec;
+        }
+        break;
+    }
     if (!exec) {
         if (graphs_.size() >= 32) {
             for (auto &g : graphs_) cudaGraphExecDestroy(g.exec);
@@ -661,7 +671,7 @@ template <class R> int Engine<R>::run_cycle(int kk, int nsys, int lead, double t
         long mv = 0;
         const bool hz = have_z_, zp = z_pending_;
         int rc = enqueue_cycle(kk, nsys, tol, &mv, true);
-        const bool untuned = set_capturing(false);
+        const CaptureTuning met = set_capturing(false);
         have_z_ = hz;
         z_pending_ = zp;
         cudaGraph_t graph = nullptr;
@@ -671,7 +681,7 @@ template <class R> int Engine<R>::run_cycle(int kk, int nsys, int lead, double t
             set_last_error(GDMR_ECUDA, std::string("restart-cycle capture: ") + cudaGetErrorString(e));
             return GDMR_ECUDA;
         }
-        if (untuned) {   // some launch's variant is not chosen yet: an eager cycle times its class
+        if (met.untuned) {   // some launch's variant is not chosen yet: an eager cycle times its class
             cudaGraphDestroy(graph);
             return enqueue_cycle(kk, nsys, tol, matvecs, false);
         }
@@ -681,7 +691,7 @@ template <class R> int Engine<R>::run_cycle(int kk, int nsys, int lead, double t
             set_last_error(GDMR_ECUDA, std::string("restart-cycle graph: ") + cudaGetErrorString(e));
             return GDMR_ECUDA;
         }
-        graphs_.push_back(GraphEntry{kk, nsys, zpar, tol, blocked, cholqr, g_direct_, exec});
+        graphs_.push_back(GraphEntry{kk, nsys, zpar, tol, blocked, cholqr, g_direct_, met.open ? generation : -1, exec});
     }
     GDMR_CK(cudaGraphLaunch(exec, stream));
     // the graph joins the deflation update into the main stream: the new Z is ready in order

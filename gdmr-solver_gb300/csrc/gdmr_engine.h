@@ -268,6 +268,7 @@ template <class R> class Engine {
         int kk, nsys, zpar;
         double tol;
         bool blocked, cholqr, gdirect;
+        int generation;   // of the tuner when a launch had no settled variant; -1: all had
         cudaGraphExec_t exec;
     };
     std::vector<GraphEntry> graphs_;

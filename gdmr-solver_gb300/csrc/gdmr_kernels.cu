@@ -5046,13 +5046,24 @@ int forced_variant(int kernel) {
     return g_forced[kernel];
 }
 thread_local bool t_capturing = false;   // a stream capture is open on this thread: no timing
-thread_local bool t_untuned = false;     // it met a class that has no variant yet
+thread_local CaptureTuning t_capture;     // what it met
+
+// The variant of a launch that is not its class's to tune; 0 while there is none.
+int settled_variant(const TuneKey &key) {
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    for (auto &e : g_tuned)
+        if (e.key == key) return e.variant;
+    if (t_capturing) t_capture.open = true;
+    return 0;
+}
 
 // One choice per (precision, kernel, n, shape class).  The shape class separates launches
 // with and without a shared segment (the deflation vectors W) and single- from multi-system
 // launches, because a batch sharing W is limited by re-reading W and favours other tiles.
 // A cycle captured into a CUDA graph holds settled classes only: one that meets an unsettled class (a
-// batch that has shrunk into another width) is not kept, and the cycle runs eagerly (Engine::run_cycle).
+// batch that has shrunk into another width) is not kept, and the cycle runs eagerly; one whose other launches
+// (the deflation loop's with fewer than 8 vectors) found no variant is captured anew once a class has been
+// settled (Engine::run_cycle).  So a process's repeat solves take the same kernels whatever came before.
 int bucket_of(int nsys, int qa, int qb) {
     // a batch against the shared vectors alone (the deflator of the blocked Krylov steps, the deflation
     // loop's Gram matrix): classes of its own by the batch, since the tensor cores' share of the time
@@ -5076,7 +5087,7 @@ int tuned_variant(int prec, int kernel, int n, int nsys, int qa, int qb, int nva
             if (e.key == key) return e.variant;
         if (!g_tune_enabled) return 0;
         if (t_capturing) {
-            t_untuned = true;
+            t_capture.untuned = true;
             return 0;
         }
     }
@@ -5120,11 +5131,17 @@ int tuned_variant(int prec, int kernel, int n, int nsys, int qa, int qb, int nva
 }
 }  // namespace
 
-bool set_capturing(bool on) {
-    const bool untuned = t_untuned;
+CaptureTuning set_capturing(bool on) {
+    const CaptureTuning met = t_capture;
     t_capturing = on;
-    t_untuned = false;
-    return untuned;
+    t_capture = CaptureTuning{};
+    return met;
+}
+int tune_generation(int n) {
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    int c = 0;
+    for (auto &e : g_tuned) c += e.key.n == n;
+    return c;
 }
 
 void tune_force(int projection, int update) {
@@ -5342,11 +5359,7 @@ int mdot_dispatch(int v, int n, const typename CT<R>::t *segA, int qa, const typ
                 launch_wproj_tc(n, qa, segA, w, strideW, act, nsys, (double *)partials, coef, strideC, st);
                 if (qb == 0) return 2;
                 int vown = 0;
-                {
-                    std::lock_guard<std::mutex> lk(g_tune_mu);
-                    for (auto &e : g_tuned)
-                        if (e.key == TuneKey{prec_key<R>(), 0, n, bucket_of(nsys, 0, 1)}) vown = e.variant;
-                }
+                vown = settled_variant(TuneKey{prec_key<R>(), 0, n, bucket_of(nsys, 0, 1)});
                 if (vown >= VW) vown = 0;
                 return 2 + mdot_dispatch<R>(vown, n, nullptr, 0, segB, strideB, qb, w, strideW, act, nsys, partials,
                                             qmax, tickets, coef + qa, strideC, state, skip_broken, st);
@@ -5367,11 +5380,7 @@ int mdot_dispatch(int v, int n, const typename CT<R>::t *segA, int qa, const typ
             if (qb == 0) return 2;
             // own-basis part: the tuned choice for a batch without a shared segment
             int vown = 0;
-            {
-                std::lock_guard<std::mutex> lk(g_tune_mu);
-                for (auto &e : g_tuned)
-                    if (e.key == TuneKey{prec_key<R>(), 0, n, bucket_of(nsys, 0, 1)}) vown = e.variant;
-            }
+            vown = settled_variant(TuneKey{prec_key<R>(), 0, n, bucket_of(nsys, 0, 1)});
             if (vown >= VW) vown = 0;
             return 2 + mdot_dispatch<R>(vown, n, nullptr, 0, segB, strideB, qb, w, strideW, act, nsys, partials, qmax,
                                         tickets, coef + qa, strideC, state, skip_broken, st);
@@ -5478,11 +5487,7 @@ void launch_mdot(int n, const typename CT<R>::t *segA, int qa, const typename CT
     int v = 0;
     if (forced_variant(0) >= 0) v = forced_variant(0);
     else if (representative(nsys, qa, qb) && !profile_enabled()) v = tuned_variant(prec_key<R>(), 0, n, nsys, qa, qb, sizeof(R) == 4 ? 11 : 14, st, run);
-    else {
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        for (auto &e : g_tuned)
-            if (e.key == TuneKey{prec_key<R>(), 0, n, bucket_of(nsys, qa, qb)}) v = e.variant;
-    }
+    else v = settled_variant(TuneKey{prec_key<R>(), 0, n, bucket_of(nsys, qa, qb)});
     run(v);
     L_.add(launched);
 }
@@ -5523,11 +5528,7 @@ int update_dispatch(int v, int n, const typename CT<R>::t *segA, int qa, const t
                 launch_wapply_tc(n, qa, segA, const_cast<double2 *>(coef), strideC, act, nsys,
                                  const_cast<typename CT<R>::t *>(segB) + (size_t)qb * n, strideB, qa + qb, st);
                 int vown = 0;
-                {
-                    std::lock_guard<std::mutex> lk(g_tune_mu);
-                    for (auto &e : g_tuned)
-                        if (e.key == TuneKey{prec_key<R>(), 1, n, bucket_of(nsys, 0, 1)}) vown = e.variant;
-                }
+                vown = settled_variant(TuneKey{prec_key<R>(), 1, n, bucket_of(nsys, 0, 1)});
                 if (vown >= VW) vown = 0;
                 return 1 + update_dispatch<R>(vown, n, nullptr, 0, segB, strideB, qb + 1, w, strideW, out, strideO,
                                               act, nsys, coef + qa, strideC, partials, tickets, state, fin,
@@ -5648,11 +5649,7 @@ void launch_update(int n, const typename CT<R>::t *segA, int qa, const typename 
     if (forced_variant(1) >= 0) v = forced_variant(1);
     else if (representative(nsys, qa, qb) && !profile_enabled())
         v = tuned_variant(prec_key<R>(), 1, n, nsys, qa, qb, sizeof(R) == 4 ? 12 : 13, st, run);
-    else {
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        for (auto &e : g_tuned)
-            if (e.key == TuneKey{prec_key<R>(), 1, n, bucket_of(nsys, qa, qb)}) v = e.variant;
-    }
+    else v = settled_variant(TuneKey{prec_key<R>(), 1, n, bucket_of(nsys, qa, qb)});
     run(v);
     L_.add(launched);
 }
@@ -5715,11 +5712,7 @@ void launch_wdeflate(int n, int kk, const float2 *W, const float2 *y, size_t str
         return;
     }
     if (nsys > 1 && !profile_enabled()) v = tuned_variant(prec_key<float>(), 2, n, nsys, kk, 0, 4, st, run);
-    else {
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        for (auto &e : g_tuned)
-            if (e.key == TuneKey{prec_key<float>(), 2, n, bucket_of(nsys, kk, 0)}) v = e.variant;
-    }
+    else v = settled_variant(TuneKey{prec_key<float>(), 2, n, bucket_of(nsys, kk, 0)});
     run(v);
 }
 

@@ -216,9 +216,15 @@ void profile_reset();
 void tune_enable(bool on);
 // Pins the projection and update variants (-1 returns each to the tuner).
 void tune_force(int projection, int update);
-// Marks the calling thread as capturing a CUDA graph: launchers then use cached choices only.  Returns whether one
-// of them has met a class without a choice since the last call.
-bool set_capturing(bool on);
+// What the launches of a capture met: a class that one of them would have tuned, or a launch that another
+// one's class has no variant for yet.
+struct CaptureTuning {
+    bool untuned = false, open = false;
+};
+// Marks the calling thread as capturing a CUDA graph: launchers then use cached choices only.  Returns what they
+// have met since the last call.  tune_generation: rises with every class of that size settled.
+CaptureTuning set_capturing(bool on);
+int tune_generation(int n);
 std::string tune_report();
 
 // ----------------------------------------------------------------- launchers

@@ -21,3 +21,21 @@ def test_a_shrinking_batch_settles_each_width_class():
     assert len({st["cycles"] for st in stats}) >= 4
     rep = [q for q in gdmr.tune_report().splitlines() if f"n={A.n} " in q and "projection" in q and "shared-only" in q]
     assert len(rep) == 4, rep
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64", "fp64e"])
+def test_repeat_solves_take_the_same_kernels_whatever_came_before(precision):
+    # the batch's graphs are captured before the single-system classes are settled, which the deflation loop's
+    # short launches share: the first system's repeat solve must match a system's that found all settled
+    A = problems.helmholtz((19, 14, 13) if precision == "mixed" else (18, 14, 13), 5.0, 0.1)
+    B = np.stack([problems.unit_gaussian_rhs(A.n, 50 + i) for i in range(2)])
+    out = []
+    for _ in range(2):
+        s = gdmr.System(A, 30, 8, capacity=2, precision=precision)
+        s.set_fused(False)
+        for _ in range(2):
+            s.drop_deflation()
+            X = s.solve_batch(B, tol=[1e-6, 1e-10], max_cycles=400)[0]
+        s.close()
+        out.append(X)
+    assert np.array_equal(out[0], out[1])
