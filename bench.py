@@ -48,11 +48,14 @@ SHAPE = (96, 96, 96)
 KAPPA, DAMPING, M, K, TOL = 24.0, 0.1, 48, 24, 1e-10
 
 
-# DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum) per algorithmic byte, per kernel
-# class, measured by ncu over three batched cycles of this same workload with the tensor-core
-# shared-basis kernels in use.
-TRAFFIC_PER_ALGORITHMIC_BYTE = {"projection": 1.027, "update": 1.043, "operator": 0.938, "combine": 1.000,
-                                "deflation_update": 1.303, "residual64": 1.478, "other": 0.949}
+# DRAM bytes (ncu) per algorithmic byte, per kernel class, and what they were captured on.  The operator
+# class has none: its kernel, k_grid_const, has not been captured.
+_CYCLES = "every launch of three cycles of this workload"
+_BLOCK = "its largest kernel, {}, at 48^3 with 64 systems and 22 basis vectors"
+TRAFFIC_PER_ALGORITHMIC_BYTE = {"projection": (1.003, _BLOCK.format("k_block_proj")),
+                                "update": (0.997, _BLOCK.format("k_block_update")), "combine": (1.000, _CYCLES),
+                                "deflation_update": (1.303, _CYCLES), "residual64": (1.478, _CYCLES),
+                                "other": (0.949, _CYCLES)}
 
 
 def peaks():
@@ -652,15 +655,14 @@ def main():
     tot_ms = sum(v["ms"] for v in prof.values())
     d = prof[dom]
     achieved = d["bytes"] / (d["ms"] / 1e3) / 1e9
-    ratio = TRAFFIC_PER_ALGORITHMIC_BYTE.get(dom)
+    ratio, captured = TRAFFIC_PER_ALGORITHMIC_BYTE.get(dom, (None, None))
     per_launch = d["bytes"] / max(1, d["launches"])
     roofline = {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                 "frac": achieved / hbm_peak, "peak_kind": peak_kind,
                 "algorithmic_bytes_per_launch": per_launch,
                 "traffic": ratio * per_launch if ratio is not None else None,
-                "traffic_basis": (f"ncu DRAM bytes = {ratio} x algorithmic bytes for this class "
-                                  "(every launch of 3 cycles of this workload), times this run's mean "
-                                  "algorithmic bytes per launch") if ratio is not None else None,
+                "traffic_basis": (f"ncu DRAM bytes = {ratio} x algorithmic bytes for this class ({captured}), times "
+                                  "this run's mean algorithmic bytes per launch") if ratio is not None else None,
                 "share": d["ms"] / tot_ms, "classes": class_table(prof, hbm_peak)}
 
     # e2e: host buffers (pinned), copies inside the timed region, through the C ABI

@@ -5987,14 +5987,16 @@ void launch_spmm(const SellMatrix &A, const typename CT<R>::t *x, size_t strideX
                  const int *act, int nsys, cudaStream_t st, const SysState *scale, typename CT<R>::t *vout,
                  size_t strideVO) {
     if (nsys <= 0) return;
-    // with the normalisation folded in, the kernel also writes v_s: one more vector a system
-    Launch L_(KC_SPMM, spmm_bytes(A, sizeof(typename CT<R>::t), nsys) +
-                           (vout ? (double)sizeof(typename CT<R>::t) * A.n * nsys : 0.0), st, 1);
-    op_mode_dispatch(scale, vout, [&](auto mode) {
-    constexpr int MODE = decltype(mode)::value;
     const int sg = nsys == 1 ? 1 : grid_batch();
     // a constant-coefficient grid operator (batches too, unless gdmrGridBatch asks for its kernel)
-    if (A.grid && A.gconst.valid && grid_operator() && (nsys == 1 || sg == 0) && nsys <= 65535) {
+    const bool planes = A.grid && A.gconst.valid && grid_operator() && (nsys == 1 || sg == 0) && nsys <= 65535;
+    // the CSR formula's bytes, or x and y alone where no coefficient is read; with the normalisation folded in,
+    // the kernel also writes v_s: one more vector a system
+    const double vec = (double)sizeof(typename CT<R>::t) * A.n * nsys;
+    Launch L_(KC_SPMM, (planes ? 2.0 * vec : spmm_bytes(A, sizeof(typename CT<R>::t), nsys)) + (vout ? vec : 0.0), st, 1);
+    op_mode_dispatch(scale, vout, [&](auto mode) {
+    constexpr int MODE = decltype(mode)::value;
+    if (planes) {
         PlaneValues<typename CT<R>::t> pv;
         for (int p = 0; p < 7; ++p) pv.a[p] = host_value<typename CT<R>::t>(A.gconst.a[p]);
         const dim3 grid(((A.gx + 31) / 32) * ((A.gy + 7) / 8), (A.gz + GR_ZC - 1) / GR_ZC, nsys);
