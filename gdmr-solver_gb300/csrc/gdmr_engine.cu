@@ -355,6 +355,7 @@ int sell_from_csr(DeviceSell &out, int n, const int *rowptr, const int *colidx, 
         }
         // constant planes: one value wherever the neighbour lies on the grid
         const int p0 = gz > 1 ? 0 : 1;                  // 7-plane index: -P, -Q, -1, 0, +1, +Q, +P
+        if (gz == 1) d.gconst.real = 0x41u;             // 2D: no planes -P and +P, so nothing complex in them
         for (int e = 0; e < np; ++e) {
             const int p = e + p0;
             const long cut = p == 0 || p == 6 ? gz : p == 1 || p == 5 ? gy : p == 2 || p == 4 ? gx : 0;
