@@ -1593,19 +1593,21 @@ __global__ void __launch_bounds__(KM_THREADS, 3) k_krylov_multi(const KrylovJob<
 // the batch (nsys x RT) is copied into shared memory with cp.async, double-buffered, in its
 // natural vector-major layout (leading dimension RT+2, so the strided thread tiling below
 // reads distinct banks).  Thread (ip, js) of row group grp accumulates the 4 x 4 outputs
-// p = ip + tilesP*a, s = js + tilesS*b over the rows grp, grp+KS, ... of each tile, and
-// converts them to double at the end.  The KS row groups are summed in shared memory
-// in a fixed order, and k_wproj_reduce sums the CTAs' partials in a fixed order.
+// p = ip + tilesP*a, s = js + tilesS*b over the rows grp, grp+KS, ... of each tile.  The KS row
+// groups are summed in shared memory in a fixed order, and k_wproj_reduce sums the CTAs' partials in a fixed order.
 constexpr int WP_KMAX = 32, WP_SMAX = 64;
-template <class R> __host__ __device__ constexpr int wp_rt() { return 32; }
+constexpr int WP_RT = 32;   // rows a tile
 
-__device__ __forceinline__ void cp_async_el(void *dst, const void *src, int bytes, bool valid) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    const int sz = valid ? bytes : 0;   // 0: zero-fill, nothing read
-    if (bytes == 8)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(sz) : "memory");
-    else
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(sz) : "memory");
+// 16- or 8-byte copies, the bytes past `bytes` zero-filled (0: nothing read)
+__device__ __forceinline__ void cp_async16z(void *dst, const void *src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async8z(void *dst, const void *src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(bytes)
+                 : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
@@ -1624,19 +1626,18 @@ __host__ __device__ inline WprojShape wproj_shape(int kk, int nsys) {
     if (w.KS > 8) w.KS = 8;
     return w;
 }
-template <class R> size_t wproj_smem(int kk, int nsys) {
+size_t wproj_smem(int kk, int nsys) {
     const WprojShape w = wproj_shape(kk, nsys);
-    const size_t tiles = 2 * (size_t)(w.KP + w.SP) * (wp_rt<R>() + 2) * sizeof(typename CT<R>::t);
+    const size_t tiles = 2 * (size_t)(w.KP + w.SP) * (WP_RT + 2) * sizeof(double2);
     const size_t red = (size_t)NT * 16 * sizeof(double2);
     return tiles > red ? tiles : red;
 }
 
-template <class R>
-__global__ void __launch_bounds__(NT, 2) k_wproj(int n, int kk, const typename CT<R>::t *__restrict__ W,
-                                                 const typename CT<R>::t *__restrict__ Y0, size_t strideY,
+__global__ void __launch_bounds__(NT, 2) k_wproj(int n, int kk, const double2 *__restrict__ W,
+                                                 const double2 *__restrict__ Y0, size_t strideY,
                                                  const int *__restrict__ act, int nsys, double *__restrict__ part) {
-    using C = typename CT<R>::t;
-    constexpr int RT = wp_rt<R>(), LD = RT + 2;
+    using C = double2;
+    constexpr int RT = WP_RT, LD = RT + 2;
     extern __shared__ __align__(16) unsigned char wp_sm[];
     __shared__ int s_act[WP_SMAX];
     const WprojShape sh = wproj_shape(kk, nsys);
@@ -1657,23 +1658,20 @@ __global__ void __launch_bounds__(NT, 2) k_wproj(int n, int kk, const typename C
         for (int e = tid; e < kk * RT; e += NT) {
             const int p = e / RT, r = e % RT;
             const bool v = r0 + r < n;
-            cp_async_el(Wt + p * LD + r, W + (size_t)p * n + (v ? r0 + r : 0), sizeof(C), v);
+            cp_async16z(Wt + p * LD + r, W + (size_t)p * n + (v ? r0 + r : 0), v ? 16 : 0);
         }
         for (int e = tid; e < nsys * RT; e += NT) {
             const int sl = e / RT, r = e % RT;
             const bool v = r0 + r < n;
-            cp_async_el(Yt + sl * LD + r, Y0 + (size_t)s_act[sl] * strideY + (v ? r0 + r : 0), sizeof(C), v);
+            cp_async16z(Yt + sl * LD + r, Y0 + (size_t)s_act[sl] * strideY + (v ? r0 + r : 0), v ? 16 : 0);
         }
         cp_async_commit();
     };
-    double2 accd[4][4];
     C acc[4][4];
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            acc[a][c] = czero<C>();
-        }
+        for (int c = 0; c < 4; ++c) acc[a][c] = czero<C>();
     int b = 0;
     if ((long)blockIdx.x < nrt) issue(blockIdx.x, 0);
     for (long rt = blockIdx.x; rt < nrt; rt += G, b ^= 1) {
@@ -1699,17 +1697,13 @@ __global__ void __launch_bounds__(NT, 2) k_wproj(int n, int kk, const typename C
         }
         __syncthreads();
     }
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) accd[a][c] = make_double2(acc[a][c].x, acc[a][c].y);
     // sum the row groups (fixed order) through shared memory, then write this CTA's partials
     double2 *red = reinterpret_cast<double2 *>(wp_sm);   // [thread][16]
     if (mine && grp > 0)
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) red[(size_t)tid * 16 + a * 4 + c] = accd[a][c];
+            for (int c = 0; c < 4; ++c) red[(size_t)tid * 16 + a * 4 + c] = acc[a][c];
     __syncthreads();
     if (mine && grp == 0) {
         for (int g = 1; g < sh.KS; ++g) {
@@ -1718,8 +1712,8 @@ __global__ void __launch_bounds__(NT, 2) k_wproj(int n, int kk, const typename C
             for (int a = 0; a < 4; ++a)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    accd[a][c].x += rg[a * 4 + c].x;
-                    accd[a][c].y += rg[a * 4 + c].y;
+                    acc[a][c].x += rg[a * 4 + c].x;
+                    acc[a][c].y += rg[a * 4 + c].y;
                 }
         }
 #pragma unroll
@@ -1729,8 +1723,8 @@ __global__ void __launch_bounds__(NT, 2) k_wproj(int n, int kk, const typename C
                 const int p = ip + sh.tilesP * a, sl = js + sh.tilesS * c;
                 if (p < kk && sl < nsys) {
                     double *pp = part + ((size_t)p * nsys + sl) * 2 * G;
-                    pp[blockIdx.x] = accd[a][c].x;
-                    pp[G + blockIdx.x] = accd[a][c].y;
+                    pp[blockIdx.x] = acc[a][c].x;
+                    pp[G + blockIdx.x] = acc[a][c].y;
                 }
             }
     }
@@ -1763,14 +1757,6 @@ __global__ void __launch_bounds__(NT) k_wproj_reduce(int kk, int nsys, int G, co
 // with chains of 128 and one tree at the end (sums off by up to 1.9e-6 of their terms, here by 1.2e-7).
 // One wave of CTAs, which chains that long could not always keep, pays for them at n = 884,736: 114 us (132).
 constexpr int WD_CH = 128, WD_ST = 3, WD_CHAIN = 8, WD_KMAX = 32, WD_WARPS = 24, WD_NT = WD_WARPS * 32;
-__device__ __forceinline__ void cp_async16z(void *dst, const void *src, int bytes) {   // zero-filled past `bytes`
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-                 "l"(src), "r"(bytes));
-}
-__device__ __forceinline__ void cp_async8z(void *dst, const void *src, int bytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-                 "l"(src), "r"(bytes));
-}
 template <int RS>
 __global__ void __launch_bounds__(WD_NT, 1) k_wdots(int n, int kk, const float2 *__restrict__ W,
                                                     const float2 *__restrict__ Y0, size_t strideY,
@@ -5242,8 +5228,8 @@ inline bool vec2_ok(int n, size_t strideB, size_t strideW) { return (n % 2 == 0)
 
 bool batched_w_ok(int kk, int nsys) { return kk > 0 && kk <= WP_KMAX && nsys >= 8 && nsys <= WP_SMAX; }
 
-int wproj_grid(int n, int rt) {
-    const long nrt = (n + rt - 1) / rt;
+int wproj_grid(int n) {
+    const long nrt = (n + WP_RT - 1) / WP_RT;
     long G = (long)num_sms() * 2;
     if (G > nrt) G = nrt;
     return G < 1 ? 1 : (int)G;
@@ -5251,13 +5237,12 @@ int wproj_grid(int n, int rt) {
 
 // Shared-W projection for a batch: two launches, no profiling bracket of its own (the
 // caller's covers it).
-template <class R>
-void wproj_run(int n, int kk, const typename CT<R>::t *W, const typename CT<R>::t *Y, size_t strideY, const int *act,
-               int nsys, double2 *partials, double2 *coef, size_t strideC, cudaStream_t st) {
-    const int G = wproj_grid(n, wp_rt<R>());
-    const size_t smem = wproj_smem<R>(kk, nsys);
-    allow_smem(k_wproj<R>, smem);
-    k_wproj<R><<<G, NT, smem, st>>>(n, kk, W, Y, strideY, act, nsys, (double *)partials);
+void wproj_run(int n, int kk, const double2 *W, const double2 *Y, size_t strideY, const int *act, int nsys,
+               double2 *partials, double2 *coef, size_t strideC, cudaStream_t st) {
+    const int G = wproj_grid(n);
+    const size_t smem = wproj_smem(kk, nsys);
+    allow_smem(k_wproj, smem);
+    k_wproj<<<G, NT, smem, st>>>(n, kk, W, Y, strideY, act, nsys, (double *)partials);
     const int outs = kk * nsys;
     k_wproj_reduce<<<(outs + NW - 1) / NW, NT, 0, st>>>(kk, nsys, G, (const double *)partials, act, coef, strideC);
 }
@@ -5372,8 +5357,8 @@ int mdot_dispatch(int v, int n, const typename CT<R>::t *segA, int qa, const typ
           bool shared = false;   // the shared part ran on its own
           if constexpr (sizeof(R) == 4) {
             shared = qa > 0 && wdots_run(n, qa, segA, w, strideW, act, nsys, partials, cap, coef, strideC, st);
-          } else if (qa > 0 && batched_w_ok(qa, nsys) && (size_t)qa * nsys * 2 * wproj_grid(n, wp_rt<R>()) <= cap) {
-            wproj_run<R>(n, qa, segA, w, strideW, act, nsys, partials, coef, strideC, st);
+          } else if (qa > 0 && batched_w_ok(qa, nsys) && (size_t)qa * nsys * 2 * wproj_grid(n) <= cap) {
+            wproj_run(n, qa, segA, w, strideW, act, nsys, partials, coef, strideC, st);
             shared = true;
           }
           if (shared) {
@@ -5974,11 +5959,12 @@ SellPattern sell_pattern(const SellMatrix &A) {
 }
 
 namespace {
-// f(OpMode constant) for a launch with these arguments (see launch_spmm)
-template <class F> void op_mode_dispatch(const SysState *scale, const void *vout, F &&f) {
+// f(OpMode constant) for a launch with these arguments (see launch_spmm); the shifted product is the blocked
+// steps', complex64's alone
+template <class R, class F> void op_mode_dispatch(const SysState *scale, const void *vout, F &&f) {
     if (!scale) f(std::integral_constant<int, OP_PLAIN>{});
     else if (vout) f(std::integral_constant<int, OP_SCALE>{});
-    else f(std::integral_constant<int, OP_SHIFT>{});
+    else if constexpr (std::is_same<R, float>::value) f(std::integral_constant<int, OP_SHIFT>{});
 }
 }  // namespace
 
@@ -5994,7 +5980,7 @@ void launch_spmm(const SellMatrix &A, const typename CT<R>::t *x, size_t strideX
     // the kernel also writes v_s: one more vector a system
     const double vec = (double)sizeof(typename CT<R>::t) * A.n * nsys;
     Launch L_(KC_SPMM, (planes ? 2.0 * vec : spmm_bytes(A, sizeof(typename CT<R>::t), nsys)) + (vout ? vec : 0.0), st, 1);
-    op_mode_dispatch(scale, vout, [&](auto mode) {
+    op_mode_dispatch<R>(scale, vout, [&](auto mode) {
     constexpr int MODE = decltype(mode)::value;
     if (planes) {
         PlaneValues<typename CT<R>::t> pv;
@@ -6052,7 +6038,7 @@ void launch_stencil(const Stencil7 &S, const typename CT<R>::t *x, size_t stride
     Launch L_(KC_SPMM, (vout ? 3.0 : 2.0) * nsys * n * sizeof(typename CT<R>::t), st, 1);
     const int tiles = ((S.nx + 31) / 32) * ((S.ny + 7) / 8);
     const dim3 grid(tiles, (S.nz + ST_ZC - 1) / ST_ZC, nsys);
-    op_mode_dispatch(scale, vout, [&](auto mode) {
+    op_mode_dispatch<R>(scale, vout, [&](auto mode) {
         using C = typename CT<R>::t;
         k_stencil<R, decltype(mode)::value><<<grid, NT, 0, st>>>(
             S.nx, S.ny, S.nz, host_value<C>(S.d), host_value<C>(S.wx), host_value<C>(S.wy), host_value<C>(S.wz), x,
