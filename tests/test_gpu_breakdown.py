@@ -159,3 +159,23 @@ def test_cholesky_factor_returns_after_a_failure():
     assert stats[0]["cycles"] > 8 and c["factor_failed"] == 1, (c, stats)
     assert c["factored"] == stats[0]["cycles"] - 4, (c, stats)
     s.close()
+
+
+def test_a_lead_that_breaks_down_leaves_the_deflation_space():
+    # one system, whose cycles from the third on are graphs: the cycle's update of the space comes from an
+    # incomplete Hessenberg and is undone, in both buffers' parities
+    A, two = _spread(N + 2)
+    s = gdmr.System(A, 30, 8, capacity=1, precision="mixed")
+    Z = _unit_vectors(A.n, 8)
+    dropped = []
+    for warm in range(4):
+        for _ in range(1 + warm % 2):
+            _check(A, _rhs(A.n, 1), *s.solve_batch(_rhs(A.n, 1), tol=TOL, max_cycles=200))
+        s.import_deflation(Z)
+        c0 = _counts()
+        stats = s.solve_batch(two[None], tol=TOL, max_cycles=1)[1]
+        dropped.append(_counts(c0)["dropped"])
+        assert stats[0]["status"] == 3 and np.array_equal(s.export_deflation(), Z)
+        _check(A, [two], *s.solve_batch(two[None], tol=TOL, max_cycles=200))
+    assert dropped == [1, 1, 1, 1]
+    s.close()
