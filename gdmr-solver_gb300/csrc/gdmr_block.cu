@@ -21,8 +21,8 @@
 // 1250 ms; 64^3, 16 systems: 663 to 515 ms; one system at 128^3, m = 60, k = 20: 655 to 612 ms.
 //
 // A block whose pivot falls below BK_ILL of its column (an exhausted or badly scaled Krylov space) sets
-// SysState::ill: the cycle's correction of that system is dropped by the caller, and the cycles after run
-// step by step.
+// SysState::ill: the caller drops the cycle's correction of that system and runs step by step while the system
+// is in flight.  (s-step bases: Chronopoulos and Gear 1989; Hoemmen 2010.)
 #include <cuda_runtime.h>
 
 #include <algorithm>

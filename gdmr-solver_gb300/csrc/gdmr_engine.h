@@ -282,9 +282,9 @@ template <class R> class Engine {
     bool blocked_ = false;
     // Cholesky QR in the deflation loop: refined_ is set around refined cycles.  A factor that breaks down
     // costs its cycle and pauses the form for CHOLQR_PAUSE cycles, whose updates replace the space, and for
-    // twice as long each time it happens again in a solve, CHOLQR_PAUSE_MAX at most: a space that stays
-    // singular costs one cycle in 65, an accident no more than a few cycles of the loop.
-    static constexpr int CHOLQR_PAUSE = 4, CHOLQR_PAUSE_MAX = 64;
+    // twice as long each time it happens again in a solve, CHOLQR_PAUSE_MAX at most: a space that comes out
+    // singular again and again costs two of 20 cycles and four of 160, an accident 16 cycles of the loop.
+    static constexpr int CHOLQR_PAUSE = 16, CHOLQR_PAUSE_MAX = 64;
     bool refined_ = false;
     int cholqr_wait_ = 0, cholqr_pause_ = CHOLQR_PAUSE;
     // The cycle's systems all start from their residuals, so the residuals' coordinates in [W V] are known
