@@ -3409,6 +3409,9 @@ __device__ __forceinline__ dfc to_dfc(double2 a) {
 // the polish went on normalised products of a phase, c and s in turn).  The vectors are the closer to
 // orthonormal for it: largest entry of V^H V - I, rms over 30 graded Hessenbergs (three decades), 1.5e-14 at
 // m = 30, k = 8, 2.1e-14 at 48, 24 and 3.6e-14 at 96, 16, against 6.1e-14, 9.5e-14 and 2.2e-13 with those.
+// Leaving the chain unnormalised costs nothing: the same form in normalised steps gives singular values and
+// vectors as far from an 80-bit Jacobi's (values 1.0e-16 to 1.7e-16 of the largest, rms, at m = 30 to 96 over three
+// and five decades; 1.0e-16 to 3.1e-16 with a phase, c and s in turn) and vectors as orthonormal.
 __device__ __forceinline__ dfr df_mul_raw(dfr a, dfr b) {
     const float p = a.hi * b.hi;
     return dfr(p, fmaf(a.hi, b.lo, fmaf(a.lo, b.hi, fmaf(a.hi, b.hi, -p))));
